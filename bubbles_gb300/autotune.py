@@ -38,7 +38,6 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 TUNED_DIR = os.path.join(HERE, "tuned")
 BLOCKS = (64, 128, 256)
 BATCHES = (2, 4, 8)
-PRUNES = (0, 1)
 PPTS = (1, 2)
 TILE_ORDERS = (0, 1)
 WORKLISTS = (0, 1, 2)
@@ -94,7 +93,7 @@ def tune_launches(g, dt, snap, steps, warm, log):
     best = dict(g.tuning())
     best_t = time_substeps(g, dt, snap, steps, warm)
     log.append({"tuning": dict(best), "seconds": best_t})
-    knobs = [("block_size", BLOCKS), ("prune", PRUNES), ("batch_pf", BATCHES), ("batch_pd", BATCHES),
+    knobs = [("block_size", BLOCKS), ("batch_pf", BATCHES), ("batch_pd", BATCHES),
              ("batch_np", BATCHES), ("particles_per_thread", PPTS), ("tile_order", TILE_ORDERS)]
     if isinstance(g, BatchSolver):
         knobs.append(("batch_worklist", WORKLISTS))

@@ -67,17 +67,29 @@ void fill_params(bbg_solver s) {
     if ((double)hi < T * (1.0 + 1e-6)) hi = nextafterf(hi, 3.4e38f);
     P.nb_lo = lo;
     P.nb_hi = hi;
-    P.h2mz = (float)T;
-    // margin of the density pass's reach test: far above the rounding of positions and cell
-    // faces (64 ulps of the largest grid coordinate) and the reference hash's 1e-4 nudge of
-    // particles on the grid's bounds
-    float cmax = 0.f;
+    // Filter of the density pass.  E bounds the error of a computed distance in units of the
+    // longest cell side: on an axis the halves of the candidate and the particle (below 2 + edge:
+    // 2^-10 and 2^-11), their difference (below 4: 2^-10) and the float rounding of the two
+    // offsets (4 ulps of the largest coordinate each).  The three fma then round by 2^-11 of at
+    // most the threshold each.
+    double side = 0, cmax = 0;
     const int dn[3] = {P.g.nx, P.g.ny, P.g.nz};
     for (int k = 0; k < 3; k++) {
-        const float top = P.g.minp[k] + (float)dn[k] * P.g.len[k];
-        cmax = fmaxf(cmax, fmaxf(fmaxf(fabsf(P.g.bmin[k]), fabsf(P.g.bmax[k])), fmaxf(fabsf(P.g.minp[k]), fabsf(top))));
+        side = std::max(side, (double)P.g.len[k]);
+        cmax = std::max(cmax, std::max(fabs((double)P.g.minp[k]), fabs((double)P.g.minp[k] + (double)dn[k] * P.g.len[k])));
     }
-    P.prune_m = fmaxf(fmaxf(1e-3f * P.h, 1.5e-4f), 64.f * cmax * 1.1920929e-7f);
+    P.filt_unit = (float)(1.0 / side);
+    for (int k = 0; k < 3; k++) P.filt_side[k] = (float)(P.g.len[k] / side);
+    const double coord = 8.0 * cmax * 1.2e-7 / side;
+    P.filt_edge = (float)(0.02 + coord);
+    const double E = std::sqrt(3.0) * (3.0 * std::ldexp(1.0, -10) + coord);
+    const double R = std::sqrt((double)hi) / side + E;
+    const double rr = R * R * (1.0 + 5.0 / 2048.0);
+    __half th = __float2half_ru((float)std::min(rr, 60000.0));
+    unsigned short tb;
+    memcpy(&tb, &th, 2);
+    P.filt = (unsigned)tb | ((unsigned)tb << 16);
+    P.h2mz = (float)T;
     const double kPi = 3.14159265358979323846;
     const float h3 = P.h2 * P.h, h4 = P.h2 * P.h2, h5 = P.h2 * h3;
     P.std_c = (float)(315.0 / (64.0 * kPi * (double)h3));
@@ -223,7 +235,7 @@ bbg_status free_all(bbg_solver s) {
     void *ptrs[] = {B.pos[0], B.pos[1], B.vel[0], B.vel[1], B.pid[0], B.pid[1], B.slot, B.force,
                     B.xstar, B.pforce, B.smoothed, B.rho, B.press, B.rhostar, B.derr, B.cell,
                     B.cell_old, B.sub, B.count, B.start, B.partials, B.tmp, B.nbr, B.st, B.stage,
-                    B.red, B.list, B.inv_rho, B.pprev, B.soa};
+                    B.red, B.list, B.inv_rho, B.pprev, B.frec};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     Prof *keep = B.prof;
@@ -913,7 +925,7 @@ bbg_status bbg_create(const bbg_solver_desc *desc, int capacity, bbg_solver *out
     ALLOC(B.rho, n); ALLOC(B.press, n); ALLOC(B.rhostar, n); ALLOC(B.derr, n);
     ALLOC(B.cell, n); ALLOC(B.cell_old, n); ALLOC(B.sub, n); ALLOC(B.tmp, n); ALLOC(B.nbr, n);
     ALLOC(B.list, (size_t)kMaxList * n); ALLOC(B.inv_rho, n); ALLOC(B.pprev, n);
-    ALLOC(B.soa, 3 * (n + 1)); B.soa_stride = n + (n & 1);
+    ALLOC(B.frec, 4 * ((n + 7) / 8));
     ALLOC(B.count, (size_t)s->cells); ALLOC(B.start, (size_t)s->cells + 1);
     ALLOC(B.partials, scan_partials_needed(s->cells));
     ALLOC(B.st, 1); ALLOC(B.stage, 6 * n); ALLOC(B.red, 4);

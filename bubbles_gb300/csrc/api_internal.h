@@ -14,6 +14,7 @@
 #include "mlp.h"
 
 #include <algorithm>
+#include <cuda_fp16.h>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>

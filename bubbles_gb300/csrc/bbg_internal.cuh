@@ -68,8 +68,12 @@ struct Params {
     float iz6;       // IsUnsafeZero(x) <=> |x| < iz6  (smallest float above 1e-6)
     float nb_lo;     // r^2 < nb_lo => IsWithinStd holds for sure
     float nb_hi;     // r^2 > nb_hi => IsWithinStd fails for sure
+    // density pass's filter in half precision, in units of the longest cell side (fill_params)
+    float filt_unit;      // 1 / that side
+    float filt_side[3];   // the cell's sides in it
+    float filt_edge;      // how far outside its cell the filter's margin covers a particle
+    unsigned filt;        // squared radius with the margin, twice, as halves
     float h2mz;      // h^2 - iz: W_std(r) > 0 <=> r^2 < h2mz (to FP32 rounding)
-    float prune_m;   // margin of the density pass's reach test (far above position rounding)
     float std_c;     // 315 / (64 pi h^3)
     float spiky_dw_c;   // 45 / (pi h^4)
     float spiky_d2w_c;  // 90 / (pi h^5)

@@ -14,7 +14,7 @@ struct Tuning {
     int batch_np = 4;      // non-pressure pass (two records per member)
     int batch_pd = 4;      // predicted-density pass
     int batch_pf = 4;      // pressure-force pass
-    int prune = 0;         // density pass: walk only the cells each particle's sphere reaches (1)
+    int prune = 0;         // accepted (0, 1), no effect: the density pass filters every candidate
     int ppt = 1;           // particles per thread of the predicted-density and pressure-force passes (1, 2)
     int tile_order = 0;    // member-walking passes: 0 block b takes tile b; 1 SM-strided (tile_of_block)
     int worklist = 1;      // batch corrector: 0 all tiles, 1 a block per listed tile, 2 persistent blocks
@@ -40,8 +40,7 @@ struct DevBufs {
     ListEntry *list;           // member lists: kMaxList entries per particle,
                                // member-major (list[q * n + i]; tile.cuh)
     float *inv_rho;            // 1 / density
-    float *soa;                // density pass: step-start x, y, z as three arrays of soa_stride
-    size_t soa_stride;
+    uint4 *frec;               // density pass: the filter's records of eight slots (k_filter_records)
     float *pprev;              // pressure of the previous substep, in the current order
     StepState *st;
     float *stage;              // n * 3 floats of staging for host copies

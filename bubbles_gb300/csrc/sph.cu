@@ -3,9 +3,9 @@
 //
 // Neighbour sets follow the reference buckets: j is a neighbour of i when
 // IsWithinStd(|x_i - x_j|, h) holds at the positions of the last grid update
-// (src/core/grid.h:423-447).  The density pass tests every candidate of the 27 cells
-// (9 contiguous slot ranges) once per substep with the exact FP32 membership test and
-// records the members in a compact list (tile.cuh); later passes walk that list.  The
+// (src/core/grid.h:423-447).  The density pass filters the candidates of the 27 cells (9
+// contiguous slot ranges) once per substep, applies the exact FP32 membership test to what
+// is left and records the members in a compact list (tile.cuh); later passes walk that list.  The
 // predicted-density pass uses the step-start membership with values at predicted
 // positions, which is what the reference does with its stale bucket
 // (src/equations/pcisph_equations3.cpp:58-89).
@@ -19,6 +19,8 @@
 // the host launches max_iterations x 2 kernels without synchronising; kernels of
 // iterations after convergence return immediately.
 #include <climits>
+
+#include <cuda_fp16.h>
 
 #include "bbg_kernels.h"
 #include "tile.cuh"
@@ -56,45 +58,11 @@ constexpr int kPfMinBlocks = BBG_PF_MIN_BLOCKS * kTile / kMaxTile;
 // spill a little)
 constexpr int kPdWlMinBlocks = BBG_PDWL_MIN_BLOCKS * kTile / kMaxTile;
 constexpr int kPfWlMinBlocks = BBG_PFWL_MIN_BLOCKS * kTile / kMaxTile;
-constexpr int kDensityMinBlocks = 12 * kTile / kMaxTile;
-#ifndef BBG_DENSITY_MASK
-#define BBG_DENSITY_MASK 1
+#ifndef BBG_DENSITY_MIN_BLOCKS
+#define BBG_DENSITY_MIN_BLOCKS 8
 #endif
-// density pass: branch-free candidate loop with membership bit masks (build-time choice;
-// measured 4 % faster than the branchy loop on GB300)
-constexpr bool kDensityMask = BBG_DENSITY_MASK != 0;
-#ifndef BBG_DENSITY_X2
-#define BBG_DENSITY_X2 1
-#endif
-// density pass on packed pairs of candidates (f32x2 arithmetic on structure-of-arrays
-// positions; build-time choice)
-constexpr bool kDensityX2 = BBG_DENSITY_X2 != 0;
-
-// Two floats in one 64-bit register pair, for the packed f32x2 instructions of sm_100+.
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 f2_pack(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2_unpack(f2 v, float &a, float &b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
-    f2 d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
-    f2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
-    f2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
+// density pass: 64 registers (measured at 1M particles: 8 and 10 blocks the same, 12 spills)
+constexpr int kDensityMinBlocks = BBG_DENSITY_MIN_BLOCKS * kTile / kMaxTile;
 
 // a neighbour's position and velocity records
 struct PosVel {
@@ -134,190 +102,38 @@ __device__ __forceinline__ bool scene_converged_before(const Params &P, int s, i
     return false;
 }
 
-// ComputeDensityFor + ComputePressureValue, src/equations/sph_equations3.cpp:7-58.
-// Tests every candidate of the 27 cells exactly once per substep and records the
-// neighbour set (the reference bucket, grid.h:423-447) as a compact member list.
-__global__ void __launch_bounds__(kMaxTile, kDensityMinBlocks)
-k_density(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, unsigned *__restrict__ cell,
-          const unsigned *__restrict__ start, float *__restrict__ rho, float *__restrict__ inv_rho,
-          float *__restrict__ press, int *__restrict__ nbr, ListEntry *__restrict__ list,
-          int compute_pressure, StepState *st) {
-    __shared__ TileMap T;
-    tile_setup(P.g, cell, start, P.n, T);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n) return;
-    const float4 pi = pos[i];
-    const unsigned cw = cell[i];
-    const size_t n = (size_t)P.n;
+// The member phase of the density pass for particle i: the exact membership test, the kernel
+// sum (i included) and the member list of candidates in the order of the 27 cells' rows, which
+// is ascending slots.  Lanes whose candidates are nearly all members write the same one or two list rows
+// together.
+struct DensitySum {
     float sum = 0.f;
-    int cnt = 0;      // bucket members, i included
     int listed = 0;   // members other than i
-    bool fits = true;
-    const bool crowded = candidate_count(P.g, start, cw & ~kWide) > kMaxCandidates;
-    if (crowded) {
-        // past the work cap: the particle itself only (counted, see kMaxCandidates)
-        sum = 1.f;
-        cnt = 1;
-        atomicAdd(&st->crowded, 1u);
-    } else if (kDensityMask) {
-        // branch-free candidate loop: membership of up to 32 consecutive candidates as a bit
-        // mask, the list entries of the members written afterwards
-        tile_rows(P.g, start, cw & ~kWide, [&](int r, unsigned b, unsigned e) {
-            const unsigned base = kListRelative ? ((unsigned)r << kOffBits) - (unsigned)T.lo[r] : 0u;
-            if (kListRelative && e - (unsigned)T.lo[r] > (unsigned)kOffLimit) fits = false;
-            for (unsigned cb = b; cb < e; cb += 32u) {
-                const unsigned ce = min(e, cb + 32u);
-                unsigned m = 0u;
-                for (unsigned j = cb; j < ce; ++j) {
-                    const float4 pj = __ldg(&pos[j]);
-                    const float r2 = dist2(pi, pj);
-                    const bool mem = r2 < P.nb_lo || (r2 <= P.nb_hi && std_member_exact(P, pi, pj));
-                    const float x = 1.f - r2 * P.inv_h2;
-                    sum += mem ? x * x * x : 0.f;
-                    m |= (unsigned)mem << (j - cb);
-                }
-                cnt += __popc(m);
-                if ((unsigned)i - cb < ce - cb) m &= ~(1u << ((unsigned)i - cb));   // the particle itself
-                while (m) {
-                    const unsigned j = cb + (unsigned)(__ffs((int)m) - 1);
-                    m &= m - 1u;
-                    if (listed < kMaxList) list[(size_t)listed * n + (size_t)i] = list_code(j, base);
-                    listed++;
-                }
-            }
-        });
-    } else tile_candidates_coded(P.g, start, T, cw & ~kWide, &fits, [&](unsigned j, unsigned base) {
-        const float4 pj = __ldg(&pos[j]);
-        const float r2 = dist2(pi, pj);
-        if (std_member(P, pi, pj, r2)) {
-            const float x = 1.f - r2 * P.inv_h2;
-            sum += x * x * x;
-            cnt++;
-            if (j != (unsigned)i) {
-                if (listed < kMaxList) list[(size_t)listed * n + (size_t)i] = list_code(j, base);
-                listed++;
-            }
-        }
-    });
+    int self = 0;     // 1 when i is its own member (not at a position that is not finite)
+    ListEntry *out;
+    __device__ __forceinline__ explicit DensitySum(ListEntry *o) : out(o) {}
+    __device__ __forceinline__ static float dist(float4 pi, float4 pj) {
+        const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+        return __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+    }
+    __device__ __forceinline__ void take(const Params &P, bool mem, float r2, unsigned j, unsigned i) {
+        const float x = __fmaf_rn(-r2, P.inv_h2, 1.f);
+        const float t = __fmul_rn(__fmul_rn(x, x), x);
+        sum = mem ? __fadd_rn(sum, t) : sum;
+        const bool other = mem && j != i;
+        if (other && listed < kMaxList) *out = j;
+        out += other ? P.n : 0;
+        listed += other ? 1 : 0;
+        self += mem && !other ? 1 : 0;
+    }
+};
+
+// The end of the density pass for particle i: density, equation of state, counters.
+__device__ __forceinline__ void density_store(const Params &P, float4 *pos, float4 *vel, unsigned *cell, float *rho,
+                                              float *inv_rho, float *press, int *nbr, int compute_pressure,
+                                              StepState *st, int i, float4 pi, unsigned cw, float sum, int cnt,
+                                              int listed) {
     const float di = sum * P.std_c * P.mass;
-    if (compute_pressure) {
-        float p = P.eos_scale_over_exp * (powf(di / P.target_density, P.eos_exp) - 1.f);
-        if (p < 0.f) p *= P.neg_scale;
-        press[i] = p;
-        reinterpret_cast<float *>(&pos[i])[3] = p / (di * di);   // pos.w = p / rho^2
-    }
-    rho[i] = di;
-    const float ir = 1.f / di;
-    inv_rho[i] = ir;
-    reinterpret_cast<float *>(&vel[i])[3] = ir;                   // vel.w = 1 / rho
-    nbr[i] = cnt;
-    if (P.nscenes > 0) P.scene[i] = (unsigned short)scene_of(P, pi.z);
-    if (listed > kMaxList || !fits) cell[i] = cw | kWide;
-    if (cnt > kBucketCap) atomicAdd(&st->nbr_overflow, 1u);
-}
-
-// Positions regrouped for the packed density pass: slots 2k and 2k + 1 share a record of six
-// floats (x of both, y of both, z of both), so a pair's coordinates are three float2 loads
-// from one address.
-__global__ void __launch_bounds__(kThreads)
-k_soa(int n, const float4 *__restrict__ pos, float *__restrict__ rec) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 p = pos[i];
-    float *r = rec + 6 * (size_t)(i >> 1) + (i & 1);
-    r[0] = p.x;
-    r[2] = p.y;
-    r[4] = p.z;
-}
-
-// k_density with candidates taken two at a time: the even-aligned pairs of each 32-candidate
-// chunk load x, y, z as float2 from the structure-of-arrays copy and compute both squared
-// distances and kernel terms with f32x2 instructions; the membership test, the running sum
-// in candidate order and the member list are those of k_density.
-__global__ void __launch_bounds__(kMaxTile, kDensityMinBlocks)
-k_density_x2(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, unsigned *__restrict__ cell,
-             const unsigned *__restrict__ start, const float *__restrict__ rec, float *__restrict__ rho,
-             float *__restrict__ inv_rho,
-             float *__restrict__ press, int *__restrict__ nbr, ListEntry *__restrict__ list, int compute_pressure,
-             StepState *st, int prune) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n) return;
-    const float4 pi = pos[i];
-    const unsigned cw = cell[i];
-    const size_t n = (size_t)P.n;
-    float s0 = 0.f;
-    int cnt = 0;      // bucket members, i included
-    int listed = 0;   // members other than i
-    // past kMaxCandidates in its 27 cells a particle is crowded: its rows stop being walked
-    // as soon as the running candidate count passes the cap (the work stays bounded), and
-    // it keeps only itself, as in k_density
-    bool crowded = false;
-    unsigned seen = 0;
-    {
-        const f2 X = f2_pack(pi.x, pi.x), Y = f2_pack(pi.y, pi.y), Z = f2_pack(pi.z, pi.z);
-        const f2 NIH = f2_pack(-P.inv_h2, -P.inv_h2), ONE = f2_pack(1.f, 1.f);
-        const float lo = P.nb_lo, hi = P.nb_hi, ih2 = P.inv_h2;
-        tile_rows_pruned(P, start, pi, cw & ~kWide, prune != 0, [&](int, unsigned b, unsigned e, unsigned whole) {
-            if (crowded) return;
-            seen += whole;   // the work cap counts the 27 cells' candidates, walked or not
-            if (seen > kMaxCandidates) {
-                crowded = true;
-                return;
-            }
-            for (unsigned cb = b; cb < e; cb += 32u) {
-                const unsigned ce = min(e, cb + 32u);
-                unsigned m = 0u;
-                unsigned j = cb;
-                auto single = [&](unsigned q) {
-                    const float *r = rec + 6 * (size_t)(q >> 1) + (q & 1u);
-                    const float4 pj = make_float4(__ldg(&r[0]), __ldg(&r[2]), __ldg(&r[4]), 0.f);
-                    const float r2 = dist2(pi, pj);
-                    const bool mem = r2 < lo || (r2 <= hi && std_member_exact(P, pi, pj));
-                    const float x = 1.f - r2 * ih2;
-                    s0 += mem ? x * x * x : 0.f;
-                    m |= (unsigned)mem << (q - cb);
-                };
-                if (j & 1u) single(j++);
-                for (; j + 1u < ce; j += 2u) {
-                    const float2 *r = reinterpret_cast<const float2 *>(rec + 3 * (size_t)j);   // j even
-                    const float2 ax = __ldg(&r[0]), ay = __ldg(&r[1]), az = __ldg(&r[2]);
-                    const f2 dx = f2_sub(f2_pack(ax.x, ax.y), X);
-                    const f2 dy = f2_sub(f2_pack(ay.x, ay.y), Y);
-                    const f2 dz = f2_sub(f2_pack(az.x, az.y), Z);
-                    const f2 r2 = f2_fma(dz, dz, f2_fma(dx, dx, f2_mul(dy, dy)));
-                    const f2 x = f2_fma(r2, NIH, ONE);
-                    const f2 x3 = f2_mul(f2_mul(x, x), x);
-                    float r0, r1, c0, c1;
-                    f2_unpack(r2, r0, r1);
-                    f2_unpack(x3, c0, c1);
-                    bool m0 = r0 < lo, m1 = r1 < lo;
-                    if ((!m0 && r0 <= hi) || (!m1 && r1 <= hi)) {   // rare: the exact test's band
-                        if (!m0 && r0 <= hi) m0 = std_member_exact(P, pi, make_float4(ax.x, ay.x, az.x, 0.f));
-                        if (!m1 && r1 <= hi) m1 = std_member_exact(P, pi, make_float4(ax.y, ay.y, az.y, 0.f));
-                    }
-                    s0 += m0 ? c0 : 0.f;   // one running sum in candidate order
-                    s0 += m1 ? c1 : 0.f;
-                    m |= ((unsigned)m0 | ((unsigned)m1 << 1)) << (j - cb);
-                }
-                if (j < ce) single(j);
-                cnt += __popc(m);
-                if ((unsigned)i - cb < ce - cb) m &= ~(1u << ((unsigned)i - cb));   // the particle itself
-                while (m) {
-                    const unsigned q = cb + (unsigned)(__ffs((int)m) - 1);
-                    m &= m - 1u;
-                    if (listed < kMaxList) list[(size_t)listed * n + (size_t)i] = list_code(q, 0u);
-                    listed++;
-                }
-            }
-        });
-    }
-    if (crowded) {
-        s0 = 1.f;
-        cnt = 1;
-        listed = 0;
-        atomicAdd(&st->crowded, 1u);
-    }
-    const float di = s0 * P.std_c * P.mass;
     if (compute_pressure) {
         float p = P.eos_scale_over_exp * (powf(di / P.target_density, P.eos_exp) - 1.f);
         if (p < 0.f) p *= P.neg_scale;
@@ -332,6 +148,229 @@ k_density_x2(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, unsig
     if (P.nscenes > 0) P.scene[i] = (unsigned short)scene_of(P, pi.z);
     if (listed > kMaxList) cell[i] = cw | kWide;
     if (cnt > kBucketCap) atomicAdd(&st->nbr_overflow, 1u);
+}
+
+// Candidates one by one (a particle whose candidates do not fit the filter's masks), counted
+// as crowded past the work cap: the particle itself only.
+__device__ __forceinline__ void density_walk(const Params &P, const float4 *__restrict__ pos,
+                                             const unsigned *__restrict__ start, unsigned c, float4 pi, unsigned i,
+                                             StepState *st, DensitySum &D) {
+    if (candidate_count(P.g, start, c) > kMaxCandidates) {
+        atomicAdd(&st->crowded, 1u);
+        D.sum = 1.f;
+        D.self = 1;
+        return;
+    }
+    tile_rows(P.g, start, c, [&](int, unsigned b, unsigned e) {
+        for (unsigned j = b; j < e; ++j) {
+            const float4 pj = __ldg(&pos[j]);
+            const float r2 = DensitySum::dist(pi, pj);
+            D.take(P, std_member(P, pi, pj, r2), r2, j, i);
+        }
+    });
+}
+
+// The member phase over `kept` non-empty masks of candidates, entry k at keep[k * stride]: (mask,
+// slot of bit 31, the next slots below it).  Four records requested together.
+__device__ __forceinline__ void density_members(const Params &P, const float4 *__restrict__ pos, float4 pi, unsigned i,
+                                                DensitySum &D, const uint2 *keep, int stride, int kept) {
+    const uint2 *const end = keep + kept * stride;
+    unsigned m = 0, base = 0;
+    while (m != 0 || keep != end) {
+        unsigned j[4];
+        bool mem[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (m == 0 && keep != end) {
+                const uint2 v = *keep;
+                m = v.x;
+                base = v.y;
+                keep += stride;
+            }
+            mem[u] = m != 0;
+            const unsigned c = (unsigned)__clz((int)m) & 31u;
+            j[u] = mem[u] ? base + c : i;
+            m &= ~(0x80000000u >> c);
+        }
+        float4 p[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) p[u] = __ldg(&pos[j[u]]);
+        float r2[4];
+        bool all = true;   // members without the exact test
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            r2[u] = DensitySum::dist(pi, p[u]);
+            all = all && r2[u] < P.nb_lo;
+        }
+        if (!all) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) mem[u] = mem[u] && std_member(P, pi, p[u], r2[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) D.take(P, mem[u], r2[u], j[u], i);
+    }
+}
+
+// Where the density pass's filter sees a particle of cell (cx, cy, cz): its offset from the
+// cell's lower corner in units of the longest cell side, or NaN when it does not lie in the cell
+// (clamped into the grid, moved since the grid update), which the filter never drops.
+__device__ __forceinline__ v3 filter_offset(const Params &P, float4 p, int cx, int cy, int cz) {
+    const GridDev &g = P.g;
+    const float x = (p.x - (g.minp[0] + (float)cx * g.len[0])) * P.filt_unit;
+    const float y = (p.y - (g.minp[1] + (float)cy * g.len[1])) * P.filt_unit;
+    const float z = (p.z - (g.minp[2] + (float)cz * g.len[2])) * P.filt_unit;
+    const float lo = -P.filt_edge, hi = P.filt_edge;
+    const bool in = x >= lo && x <= P.filt_side[0] + hi && y >= lo && y <= P.filt_side[1] + hi && z >= lo &&
+                    z <= P.filt_side[2] + hi;
+    const float nan = __int_as_float(0x7fffffff);
+    return in ? V(x, y, z) : V(nan, nan, nan);
+}
+
+__device__ __forceinline__ void cell_coords(const GridDev &g, unsigned c, int &cx, int &cy, int &cz) {
+    const unsigned plane = (unsigned)g.nx * (unsigned)g.ny;
+    cz = (int)(c / plane);
+    const unsigned rem = c - (unsigned)cz * plane;
+    cy = (int)(rem / (unsigned)g.nx);
+    cx = (int)(rem - (unsigned)cy * (unsigned)g.nx);
+}
+
+// Positions in half precision for the density pass's filter: slots 8k .. 8k + 7 share a record of
+// four rows of eight halves, x, y, z and x'.  y and z are offsets from the centre of the
+// particle's own cell; x counts cells modulo 4 from the middle of a window of four, x' with the
+// window two cells on, so that the three cells around any cell lie in one of the two windows.
+__global__ void __launch_bounds__(kThreads)
+k_filter_records(Params P, const float4 *__restrict__ pos, const unsigned *__restrict__ cell, __half *__restrict__ rec) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P.n) return;
+    int cx, cy, cz;
+    cell_coords(P.g, cell[i] & ~kWide, cx, cy, cz);
+    const v3 f = filter_offset(P, pos[i], cx, cy, cz);
+    __half *r = rec + 32 * (size_t)(i >> 3) + (i & 7);
+    r[0] = __float2half_rn((float)((cx & 3) - 2) * P.filt_side[0] + f.x);
+    r[8] = __float2half_rn(f.y - 0.5f * P.filt_side[1]);
+    r[16] = __float2half_rn(f.z - 0.5f * P.filt_side[2]);
+    r[24] = __float2half_rn((float)(((cx + 2) & 3) - 2) * P.filt_side[0] + f.x);
+}
+
+__device__ __forceinline__ unsigned half2_bits(__half2 v) { return *reinterpret_cast<unsigned *>(&v); }
+__device__ __forceinline__ __half2 as_half2(unsigned v) { return *reinterpret_cast<__half2 *>(&v); }
+
+// Masks a particle keeps between the filter and the member phase of k_density_mask: 9 rows and
+// one more for a row whose slots span more than 32.
+constexpr int kMasks = 10;
+
+// The density pass: ComputeDensityFor + ComputePressureValue (sph_equations3.cpp:7-58), and each
+// particle's neighbour set (the reference bucket, grid.h:423-447) as a member list.  A thread per
+// particle, in two phases.
+//
+// Filter: all candidates of the 27 cells (about 216), eight at a time from k_filter_records' halves:
+// the sign of P.filt - r^2, the squared radius widened by the rounding of the halves, into a
+// mask of 32 aligned slots, and nothing else.  It only leaves out what cannot be a member.
+// Members: the exact test, the kernel sum in float and the list over the about 29 candidates left.
+//
+// Measured at 1,048,576 particles (with the records' launch): 234 -> 156 us; 4,194,304: 866 -> 578;
+// 262,144: 78 -> 52.  The pass that tested and summed every candidate in float was bound by issue
+// slots (256 M warp instructions, 83 %); this one issues 136 M.  The filter's bound is the FMA
+// pipe (24 half2 operations per eight candidates); with float candidates it was L1, whose 128 bytes
+// a clock return 12 bytes a candidate to every lane (181 us), half of that as halves.  A warp per
+// cell that holds candidates in registers and ballots each particle's tests was slower (225 us): the
+// setup per cell, 5.5 cells a warp, costs more than the loads it saves.
+__global__ void __launch_bounds__(kMaxTile, kDensityMinBlocks)
+k_density_mask(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, unsigned *__restrict__ cell,
+               const unsigned *__restrict__ start, const uint4 *__restrict__ rec, float *__restrict__ rho,
+               float *__restrict__ inv_rho, float *__restrict__ press, int *__restrict__ nbr,
+               ListEntry *__restrict__ list, int compute_pressure, StepState *st) {
+    extern __shared__ uint2 mask_smem[];   // [kMasks][blockDim.x]: mask, slot of its bit 31
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P.n) return;
+    uint2 *const keep = mask_smem + threadIdx.x;
+    const int stride = (int)blockDim.x;
+    const float4 pi = pos[i];
+    const unsigned cw = cell[i], c = cw & ~kWide;
+    int kept = 0;
+    unsigned total = 0;
+    {
+        const GridDev &g = P.g;
+        int cx, cy, cz;
+        cell_coords(g, c, cx, cy, cz);
+        const v3 f = filter_offset(P, pi, cx, cy, cz);
+        const int far = ((cx + 1) & 2) ? 0 : 1;   // cells 1 and 2 of the first window, else the second
+        const __half2 X = __float2half2_rn((float)(((cx + 2 * far) & 3) - 2) * P.filt_side[0] + f.x);
+        const __half2 T = as_half2(P.filt);
+        // rows x, y, z of a record, or y, z, x' of the second window: the test takes the axes in any order
+        const uint4 *const rec0 = rec + far;
+        const int x0 = cx > 0 ? -1 : 0, x1 = cx + 1 < g.nx ? 2 : 1;
+        const int plane = g.nx * g.ny;
+        // row r = 3 (dz + 1) + dy + 1, inside the grid or empty; the next row's range is requested a row ahead
+        unsigned inside = 0x1ffu;
+        if (cy == 0) inside &= ~0x049u;
+        if (cy + 1 >= g.ny) inside &= ~0x124u;
+        if (cz == 0) inside &= ~0x007u;
+        if (cz + 1 >= g.nz) inside &= ~0x1c0u;
+        int row = (int)c - g.nx - plane;
+        unsigned nb = 0, ne = 0;
+        if (inside & 1u) {
+            nb = __ldg(&start[row + x0]);
+            ne = __ldg(&start[row + x1]);
+        }
+        __half2 Z = __float2half2_rn(f.z + 0.5f * P.filt_side[2]);
+        float fy = f.y + 0.5f * P.filt_side[1];
+        int dy = 0;
+#pragma unroll 1
+        for (int r = 0; r < 9; r++) {
+            const unsigned b = nb, e = ne;
+            const __half2 Y = __float2half2_rn(fy);
+            const __half2 A = far ? Y : X, B = far ? Z : Y, C = far ? X : Z;
+            fy -= P.filt_side[1];
+            row += g.nx;
+            if (++dy == 3) {
+                dy = 0;
+                row += plane - 3 * g.nx;
+                fy = f.y + 0.5f * P.filt_side[1];
+                Z = __float2half2_rn(f.z + (r == 2 ? -0.5f : -1.5f) * P.filt_side[2]);
+            }
+            inside >>= 1;
+            nb = ne = 0;
+            if (inside & 1u) {
+                nb = __ldg(&start[row + x0]);
+                ne = __ldg(&start[row + x1]);
+            }
+            total += e - b;
+            for (unsigned cb = b & ~7u; cb < e; cb += 32u) {
+                const unsigned span = min(32u, e - cb);
+                const int groups = (int)((span + 7u) >> 3);
+                const uint4 *q = rec0 + (size_t)(cb >> 3) * 4u;
+                unsigned m = 0;
+                for (int k = 0; k < groups; k++, q += 4) {
+                    const uint4 a = __ldg(q), v = __ldg(q + 1), w = __ldg(q + 2);
+                    auto test = [&](unsigned ua, unsigned ub, unsigned uc) {
+                        const __half2 da = __hsub2(as_half2(ua), A), db = __hsub2(as_half2(ub), B);
+                        const __half2 dc = __hsub2(as_half2(uc), C);
+                        return half2_bits(__hfma2(__hneg2(da), da, __hfma2(__hneg2(db), db, __hfma2(__hneg2(dc), dc, T))));
+                    };
+                    const unsigned w0 = test(a.x, v.x, w.x), w1 = test(a.y, v.y, w.y);
+                    const unsigned w2 = test(a.z, v.z, w.z), w3 = test(a.w, v.w, w.w);
+                    // the eight signs (set: outside) as a byte, the first slot its top bit
+                    unsigned s = __dp4a(__byte_perm(w0, w1, 0x7531) & 0x80808080u, 0x10204080u, 0u);
+                    s = __dp4a(__byte_perm(w2, w3, 0x7531) & 0x80808080u, 0x01020408u, s);
+                    m = (m << 8) + (s >> 7);
+                }
+                m = ~m << (32 - 8 * groups);
+                // the slots of [b, e) only
+                if (b > cb) m &= 0xffffffffu >> (b - cb);
+                m &= (unsigned)((int)0x80000000 >> (span - 1u));
+                if (m) {
+                    if (kept < kMasks) keep[kept * stride] = make_uint2(m, cb);
+                    kept++;
+                }
+            }
+        }
+    }
+    DensitySum D(list + i);
+    if (kept > kMasks || total > kMaxCandidates) density_walk(P, pos, start, c, pi, (unsigned)i, st, D);
+    else density_members(P, pos, pi, (unsigned)i, D, keep, stride, kept);
+    density_store(P, pos, vel, cell, rho, inv_rho, press, nbr, compute_pressure, st, i, pi, cw, D.sum,
+                  D.listed + D.self, D.listed);
 }
 
 // ComputeNonPressureForceFor (sph_equations3.cpp:80-110), optionally followed by the
@@ -351,8 +390,6 @@ k_non_pressure(Params P, const float4 *__restrict__ pos, const float4 *__restric
                float *__restrict__ press, float *__restrict__ divsum, int predict, float dt, float dt_over_m) {
     const int s0 = tile_of_block(P, blockIdx.x, (P.n + (int)blockDim.x - 1) / (int)blockDim.x) * blockDim.x;
     if (s0 >= P.n) return;
-    __shared__ TileMap T;
-    tile_setup_at(P.g, cell, start, s0, T);
     const int i = s0 + threadIdx.x;
     if (i >= P.n) return;
     const float4 pi = pos[i];
@@ -366,7 +403,7 @@ k_non_pressure(Params P, const float4 *__restrict__ pos, const float4 *__restric
     const float kv = P.visc_m2 * P.spiky_d2w_c;
     const float kg = P.m2 * P.spiky_dw_c;
     tile_members<NB>(
-        P, start, T, list, nbr, pos, cell[i], i,
+        P, start, list, nbr, pos, cell[i], i,
         [&](unsigned j) { return PosVel{__ldg(&pos[j]), __ldg(&vel[j])}; },
         [&](const PosVel &nb) {
             const float4 pj = nb.p, vj = nb.v;   // vj.w = 1 / rho_j
@@ -464,7 +501,7 @@ __global__ void k_pack_acoef(int n, float4 *pos, const float *__restrict__ press
 template <int NB>
 __device__ __forceinline__ float pred_density_one(const Params &P, float4 *pos, const float4 *__restrict__ xstar,
                                                   const unsigned *__restrict__ cell,
-                                                  const unsigned *__restrict__ start, const TileMap &T,
+                                                  const unsigned *__restrict__ start,
                                                   const ListEntry *__restrict__ list,
                                                   const int *__restrict__ nbr, float *__restrict__ press,
                                                   float *__restrict__ rhostar, float *__restrict__ derr, int k,
@@ -479,7 +516,7 @@ __device__ __forceinline__ float pred_density_one(const Params &P, float4 *pos, 
         const float4 xi = xstar[i];
         float sum = 1.f;   // the particle itself: W_std(0) / (315 / (64 pi h^3))
         tile_members<NB, true>(
-            P, start, T, list, nbr, pos, cell[i], i, [&](unsigned j) { return __ldg(&xstar[j]); },
+            P, start, list, nbr, pos, cell[i], i, [&](unsigned j) { return __ldg(&xstar[j]); },
             [&](const float4 xj) {
                 const float r2 = dist2(xi, xj);
                 if (r2 < P.h2mz) {
@@ -610,14 +647,12 @@ k_pred_density(Params P, float4 *pos, const float4 *__restrict__ xstar,
     if (!corrector_iteration(P, st, k)) return;
     const int s0 = block_tile(P, wl, PPT * blockDim.x);
     if (s0 < 0 || s0 >= P.n) return;
-    __shared__ TileMap T;
     float amax = 0.f, asum = 0.f;
 #pragma unroll 1
     for (int u = 0; u < PPT; u++) {
         const int su = s0 + u * blockDim.x;
-        tile_setup_at(P.g, cell, start, su < P.n ? su : s0, T);
         int sc;
-        const float aerr = pred_density_one<NB>(P, pos, xstar, cell, start, T, list, nbr, press, rhostar, derr,
+        const float aerr = pred_density_one<NB>(P, pos, xstar, cell, start, list, nbr, press, rhostar, derr,
                                                 k, delta, clamp_total, su + threadIdx.x, sc);
         amax = fmaxf(amax, aerr);
         asum += aerr;
@@ -636,7 +671,6 @@ k_pred_density_wl(Params P, float4 *pos, const float4 *__restrict__ xstar,
                   float *__restrict__ rhostar, float *__restrict__ derr, StepState *st, int k,
                   float delta, int clamp_total) {
     if (!corrector_iteration(P, st, k)) return;
-    __shared__ TileMap T;
     __shared__ int slot[2];
     int parity = 0;
     const int total = worklist_total(P, blockDim.x);
@@ -646,9 +680,8 @@ k_pred_density_wl(Params P, float4 *pos, const float4 *__restrict__ xstar,
         if (w >= total) break;
         const int s0 = worklist_tile(P, w) * blockDim.x;
         if (s0 < 0 || s0 >= P.n) continue;   // never for a list built by k_worklist
-        tile_setup_at(P.g, cell, start, s0, T);
         int sc;
-        const float aerr = pred_density_one<NB>(P, pos, xstar, cell, start, T, list, nbr, press, rhostar, derr,
+        const float aerr = pred_density_one<NB>(P, pos, xstar, cell, start, list, nbr, press, rhostar, derr,
                                                 k, delta, clamp_total, s0 + threadIdx.x, sc);
         amax = fmaxf(amax, aerr);
         asum += aerr;
@@ -664,7 +697,7 @@ template <int NB>
 __device__ __forceinline__ void pressure_force_one(const Params &P, const float4 *__restrict__ pos,
                                                    const float4 *__restrict__ vel,
                                                    const unsigned *__restrict__ cell,
-                                                   const unsigned *__restrict__ start, const TileMap &T,
+                                                   const unsigned *__restrict__ start,
                                                    const ListEntry *__restrict__ list,
                                                    const int *__restrict__ nbr, float4 *__restrict__ force,
                                                    float4 *__restrict__ pforce, float4 *__restrict__ xstar,
@@ -685,7 +718,7 @@ __device__ __forceinline__ void pressure_force_one(const Params &P, const float4
     float tx = 0.f, ty = 0.f, tz = 0.f;
     const float kg = P.m2 * P.spiky_dw_c;
     tile_members<NB>(
-        P, start, T, list, nbr, pos, cell[i], i, [&](unsigned j) { return __ldg(&pos[j]); },
+        P, start, list, nbr, pos, cell[i], i, [&](unsigned j) { return __ldg(&pos[j]); },
         [&](const float4 pj) {   // pj.w = p_j / rho*_j^2
             const float r2 = dist2(pi, pj);
             const float inv_d = rsqrtf(r2);
@@ -736,14 +769,12 @@ k_pressure_force(Params P, const float4 *__restrict__ pos, const float4 *__restr
     const bool last = corrector_ends(P, st, k, max_it, mode);
     const int s0 = block_tile(P, wl, PPT * blockDim.x);
     if (s0 < 0 || s0 >= P.n) return;
-    __shared__ TileMap T;
     unsigned fbits = 0;
     bool bad = false;   // integrated position or velocity not finite
 #pragma unroll 1
     for (int u = 0; u < PPT; u++) {
         const int su = s0 + u * blockDim.x;
-        tile_setup_at(P.g, cell, start, su < P.n ? su : s0, T);
-        pressure_force_one<NB>(P, pos, vel, cell, start, T, list, nbr, force, pforce, xstar, pos_out, vel_out,
+        pressure_force_one<NB>(P, pos, vel, cell, start, list, nbr, force, pforce, xstar, pos_out, vel_out,
                                k, max_it, dt, dt_over_m, mode, last, su + threadIdx.x, fbits, bad);
     }
     fbits = warp_max_u(fbits);
@@ -761,7 +792,6 @@ k_pressure_force_wl(Params P, const float4 *__restrict__ pos, const float4 *__re
                     float4 *__restrict__ vel_out, StepState *st, int k, int max_it, float dt, float dt_over_m,
                     int mode) {
     if (!corrector_iteration(P, st, k)) return;
-    __shared__ TileMap T;
     __shared__ int slot[2];
     int parity = 0;
     const int total = worklist_total(P, blockDim.x);
@@ -772,8 +802,7 @@ k_pressure_force_wl(Params P, const float4 *__restrict__ pos, const float4 *__re
         if (w >= total) break;
         const int s0 = worklist_tile(P, w) * blockDim.x;
         if (s0 < 0 || s0 >= P.n) continue;   // never for a list built by k_worklist
-        tile_setup_at(P.g, cell, start, s0, T);
-        pressure_force_one<NB>(P, pos, vel, cell, start, T, list, nbr, force, pforce, xstar, pos_out, vel_out, k,
+        pressure_force_one<NB>(P, pos, vel, cell, start, list, nbr, force, pforce, xstar, pos_out, vel_out, k,
                                max_it, dt, dt_over_m, mode, false, s0 + threadIdx.x, fbits, bad);
     }
     fbits = warp_max_u(fbits);
@@ -886,8 +915,6 @@ k_sph_forces(Params P, const float4 *__restrict__ pos, const float4 *__restrict_
              const unsigned *__restrict__ cell, const unsigned *__restrict__ start,
              const ListEntry *__restrict__ list, const int *__restrict__ nbr, float4 *__restrict__ force,
              float4 *__restrict__ pos_out, float4 *__restrict__ vel_out, StepState *st, float dt) {
-    __shared__ TileMap T;
-    tile_setup(P.g, cell, start, P.n, T);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned fbits = 0;
     bool bad = false;   // integrated position or velocity not finite
@@ -902,7 +929,7 @@ k_sph_forces(Params P, const float4 *__restrict__ pos, const float4 *__restrict_
         const float kg = P.m2 * P.spiky_dw_c;
         const float kv = P.visc_m2 * P.spiky_d2w_c;
         tile_members<(kGatherBatch < 4 ? kGatherBatch : 4)>(
-            P, start, T, list, nbr, pos, cell[i], i,
+            P, start, list, nbr, pos, cell[i], i,
             [&](unsigned j) { return PosVel{__ldg(&pos[j]), __ldg(&vel[j])}; },
             [&](const PosVel &nb) {
                 const float4 pj = nb.p, vj = nb.v;   // vj.w = 1 / rho_j
@@ -973,8 +1000,6 @@ k_pv_aggregate(Params P, const float4 *__restrict__ pos_old, const float4 *__res
                const float4 *__restrict__ vel, const float *__restrict__ inv_rho,
                const unsigned *__restrict__ cell, const unsigned *__restrict__ start,
                const ListEntry *__restrict__ list, const int *__restrict__ nbr, float4 *__restrict__ smoothed) {
-    __shared__ TileMap T;
-    tile_setup(P.g, cell, start, P.n, T);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
     const float4 pi = pos[i];
@@ -983,7 +1008,7 @@ k_pv_aggregate(Params P, const float4 *__restrict__ pos_old, const float4 *__res
     const float4 v0 = vel[i];
     float ws = w0, sx = w0 * v0.x, sy = w0 * v0.y, sz = w0 * v0.z;
     tile_members(
-        P, start, T, list, nbr, pos_old, cell[i], i, [&](unsigned j) { return j; },
+        P, start, list, nbr, pos_old, cell[i], i, [&](unsigned j) { return j; },
         [&](unsigned j) {
             const float4 pj = __ldg(&pos[j]);
             const float d = sqrtf(dist2(pi, pj));
@@ -1024,15 +1049,13 @@ k_export_members(Params P, const unsigned *__restrict__ cell, const unsigned *__
                  const ListEntry *__restrict__ list, const int *__restrict__ nbr,
                  const float4 *__restrict__ pos0, const int *__restrict__ pid, int a, int b, int maxm,
                  int *__restrict__ counts, int *__restrict__ out) {
-    __shared__ TileMap T;
-    tile_setup(P.g, cell, start, P.n, T);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
     const int id = pid[i];
     if (id < a || id >= b) return;
     int *row = out + (size_t)(id - a) * (size_t)maxm;
     int c = 0;
-    tile_members<1>(P, start, T, list, nbr, pos0, cell[i], i, [&](unsigned j) { return j; },
+    tile_members<1>(P, start, list, nbr, pos0, cell[i], i, [&](unsigned j) { return j; },
                     [&](unsigned j) {
                         if (c < maxm) row[c] = pid[j];
                         c++;
@@ -1050,15 +1073,11 @@ void launch_export_members(const Params &P, const DevBufs &B, int buf, int pid_b
 void launch_density(const Params &P, const DevBufs &B, int buf, int compute_pressure, cudaStream_t s) {
     BBG_PBEGIN(B, KID_DENSITY, s, -1);
     const int t = B.tune.block;
-    if (kDensityX2 && !kListRelative) {
-        k_soa<<<blocks_for(P.n, kThreads), kThreads, 0, s>>>(P.n, B.pos[buf], B.soa);
-        k_density_x2<<<blocks_for(P.n, t), t, 0, s>>>(P, B.pos[buf], B.vel[buf], B.cell, B.start, B.soa, B.rho,
-                                                      B.inv_rho, B.press, B.nbr, B.list, compute_pressure, B.st,
-                                                      B.tune.prune);
-    } else {
-        k_density<<<blocks_for(P.n, t), t, 0, s>>>(P, B.pos[buf], B.vel[buf], B.cell, B.start, B.rho, B.inv_rho,
-                                                   B.press, B.nbr, B.list, compute_pressure, B.st);
-    }
+    k_filter_records<<<blocks_for(P.n, kThreads), kThreads, 0, s>>>(P, B.pos[buf], B.cell,
+                                                                    reinterpret_cast<__half *>(B.frec));
+    k_density_mask<<<blocks_for(P.n, t), t, sizeof(uint2) * kMasks * (size_t)t, s>>>(
+        P, B.pos[buf], B.vel[buf], B.cell, B.start, B.frec, B.rho, B.inv_rho, B.press, B.nbr, B.list,
+        compute_pressure, B.st);
     if (P.nscenes > 0 && P.n > 0) {
         // batch: each scene's slot range (the scene of every slot was set just above)
         cudaMemsetAsync(P.scene_first, 0x7f, sizeof(int) * (size_t)P.nscenes, s);
@@ -1144,9 +1163,8 @@ void update_worklist_grid(DevBufs &B) {
     B.tune.wl_grid_pf = B.tune.batch_pf == 2 ? pf_grid<2>(t) : B.tune.batch_pf == 8 ? pf_grid<8>(t) : pf_grid<4>(t);
 }
 
-// Particles per thread of the per-tile corrector passes (1 with tile-relative lists,
-// whose entries are decoded against the block's own tile).
-static int corrector_ppt(const DevBufs &B) { return kListRelative ? 1 : (B.tune.ppt == 2 ? 2 : 1); }
+// Particles per thread of the per-tile corrector passes.
+static int corrector_ppt(const DevBufs &B) { return B.tune.ppt == 2 ? 2 : 1; }
 
 // Slots per tile of the corrector passes: the block, times the particles per thread for
 // the per-tile kernels.

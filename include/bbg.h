@@ -468,8 +468,7 @@ bbg_status bbg_marching_cubes(bbg_solver s, const bbg_sdf_grid *grid, const floa
 /* ----- launch tuning ------------------------------------------------------------ */
 /* Block size of the neighbour passes (each block walks one tile of consecutive cell-
  * sorted particles), how many members' records a thread requests together in the
- * non-pressure, predicted-density and pressure-force passes, and whether the density pass
- * leaves out the neighbour cells (and rows of cells) a particle's sphere cannot reach.
+ * non-pressure, predicted-density and pressure-force passes.
  * Results do not depend on them (bit for bit); bubbles_gb300.autotune measures and picks
  * them. */
 typedef struct {
@@ -477,7 +476,7 @@ typedef struct {
     int batch_np;        /* 2, 4 (default) or 8 */
     int batch_pd;
     int batch_pf;
-    int prune;           /* 0 (default: measured faster on GB300) or 1 */
+    int prune;           /* 0 or 1; no effect (the density pass filters all 27 cells' candidates) */
     int particles_per_thread;  /* predicted-density and pressure-force passes: 1 (default) or 2 */
     int tile_order;      /* member-walking passes: 0 (default) block b takes tile b; 1 blocks
                             b, b + S, b + 2S, ... (S = the SM count) take consecutive tiles */
