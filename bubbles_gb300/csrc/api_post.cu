@@ -199,7 +199,8 @@ bbg_status bbg_collider_query(bbg_solver s, int index, int n, const float *point
 // ----------------------------------------------------------------------------
 namespace {
 
-// Node values of the mesh's field into device memory (*values, owned by the caller).
+// Node values of the mesh's field into device memory (*values, owned by the caller); with
+// values = nullptr the mesh is checked and the field's grid filled in, nothing computed.
 bbg_status mesh_field(bbg_solver s, const float *vertices, int nv, const int *triangles, int nt, double dx,
                       double margin, bbg_sdf_grid *g, float **values, int *stuck) {
     if (!vertices || !triangles || nv < 3 || nt < 1) return fail(BBG_ERR_INVALID_ARGUMENT, "need a mesh");
@@ -227,6 +228,7 @@ bbg_status mesh_field(bbg_solver s, const float *vertices, int nv, const int *tr
         g->bounds_min[k] = lo[k];
         g->bounds_max[k] = hi[k];
     }
+    if (!values) return BBG_OK;
     // gamma(n) = n eps / (1 - n eps) with the reference's MachineEpsilon, in double
     float gam[4];
     const int ns[4] = {2, 3, 5, 7};
@@ -236,29 +238,33 @@ bbg_status mesh_field(bbg_solver s, const float *vertices, int nv, const int *tr
     // tiles of consecutive triangles with their boxes; the distance margin is 1e-3 of the
     // mesh's bounding diagonal
     const size_t ntile = (size_t)mesh_tiles(nt);
-    std::vector<float> tiles(6 * ntile), dtri(9 * (size_t)nt), dtiles(6 * ntile);
+    std::vector<float> tiles(8 * ntile), dtri(9 * (size_t)nt), dtiles(8 * ntile);
     mesh_tile_bounds(tri.data(), nt, tiles.data());
     mesh_morton_order(tri.data(), nt, lo, hi, dtri.data());
     mesh_tile_bounds(dtri.data(), nt, dtiles.data());
     const double ex = (double)hi[0] - lo[0], ey = (double)hi[1] - lo[1], ez = (double)hi[2] - lo[2];
     const float margin_abs = (float)(1e-3 * std::sqrt(ex * ex + ey * ey + ez * ez));
-    // one upload: triangles, their tiles, the Morton-ordered triangles, their tiles
-    tri.insert(tri.end(), tiles.begin(), tiles.end());
-    tri.insert(tri.end(), dtri.begin(), dtri.end());
-    tri.insert(tri.end(), dtiles.begin(), dtiles.end());
-    float *d_tri = nullptr, *d_out = nullptr;
+    // one upload: the tiles' boxes (read as float4), the Morton-ordered triangles' boxes, the
+    // triangles in both orders
+    std::vector<float> up(tiles);
+    up.insert(up.end(), dtiles.begin(), dtiles.end());
+    up.insert(up.end(), tri.begin(), tri.end());
+    up.insert(up.end(), dtri.begin(), dtri.end());
+    const float least[2] = {float_above(1e-8), float_above(0.0001)};
+    float *d_up = nullptr, *d_rec = nullptr, *d_out = nullptr;
     unsigned *d_stuck = nullptr;
     cudaError_t e = scratch_begin(s);
-    if (e == cudaSuccess) e = scratch_get(s, tri.size(), &d_tri);
+    if (e == cudaSuccess) e = scratch_get(s, up.size(), &d_up);
+    if (e == cudaSuccess) e = scratch_get(s, mesh_record_floats(nt), &d_rec);
     if (e == cudaSuccess) e = scratch_get(s, 1, &d_stuck);
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_out, sizeof(float) * total);   // the field: the caller's
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_tri, tri.data(), sizeof(float) * tri.size(), cudaMemcpyHostToDevice, s->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_up, up.data(), sizeof(float) * up.size(), cudaMemcpyHostToDevice, s->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_stuck, 0, sizeof(unsigned), s->stream);
     unsigned h_stuck = 0;
     if (e == cudaSuccess) {
-        const float *d_tiles = d_tri + 9 * (size_t)nt, *d_dtri = d_tiles + 6 * ntile;
-        launch_mesh_sdf(d_tri, nt, d_tiles, d_dtri, d_dtri + 9 * (size_t)nt, margin_abs, field_dev(*g, d_out), lo, hi,
-                        gam, d_out, d_stuck, s->stream);
+        const float *d_dtiles = d_up + 8 * ntile, *d_tri = d_dtiles + 8 * ntile;
+        launch_mesh_sdf(d_tri, nt, d_up, d_tri + 9 * (size_t)nt, d_dtiles, margin_abs, field_dev(*g, d_out), lo, hi, gam,
+                        least, d_rec, d_out, d_stuck, s->stream);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_stuck, d_stuck, sizeof(unsigned), cudaMemcpyDeviceToHost, s->stream);
@@ -280,7 +286,9 @@ bbg_status bbg_mesh_sdf(bbg_solver s, const float *vertices, int nv, const int *
     if (bbg_status r = check_solver(s)) return r;
     bbg_sdf_grid g;
     float *d = nullptr;
-    if (bbg_status r = mesh_field(s, vertices, nv, triangles, nt, dx, margin, &g, &d, stuck)) return r;
+    // a size query (neither values nor the stuck count asked for) needs no field
+    if (bbg_status r = mesh_field(s, vertices, nv, triangles, nt, dx, margin, &g, values || stuck ? &d : nullptr, stuck))
+        return r;
     const size_t total = (size_t)g.nodes[0] * g.nodes[1] * g.nodes[2];
     if (grid) *grid = g;
     if (count) *count = total;

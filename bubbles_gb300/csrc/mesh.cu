@@ -12,6 +12,10 @@
 // are the reference's except where two triangles tie for the closest hit (the reference's
 // BVH order picks one of them, here the last by index does).  Triangles are read by all
 // threads of a warp together (broadcast loads through L1).
+//
+// FP64 runs at 1/64 of the FP32 rate here, so nothing of a triangle alone is computed per node:
+// k_mesh_records does the reference's double cross products once a triangle, and the
+// double comparisons with constants are float comparisons with the least float above them.
 #include "bbg_internal.cuh"
 #include "bbg_kernels.h"
 
@@ -25,11 +29,6 @@ static inline int blocks_for(long long n, int t) { return (int)((n + t - 1) / t)
 
 namespace {
 
-__device__ __forceinline__ v3 tri_vertex(const float *__restrict__ tri, int t, int k) {
-    const float *p = tri + 9 * (size_t)t + 3 * k;
-    return V(__ldg(p), __ldg(p + 1), __ldg(p + 2));
-}
-
 __device__ __forceinline__ float sgn(float a) { return a > 0.f ? 1.f : (a < 0.f ? -1.f : 0.f); }
 
 // Cross in double, rounded to float per component (geometry.h:906-914)
@@ -40,32 +39,71 @@ __device__ __forceinline__ v3 cross_d(v3 a, v3 b) {
              __double2float_rn(__dsub_rn(__dmul_rn(ax, by), __dmul_rn(ay, bx))));
 }
 
-// Clamp(v, 0.0001, 1.0) with the double bounds returned as floats
-__device__ __forceinline__ float clamp_edge(float v) {
-    if ((double)v < 0.0001) return 0.0001f;
-    if ((double)v > 1.0) return 1.f;
+// Clamp(v, 0.0001, 1.0) with the double bounds returned as floats; below: the least float
+// that is not below 0.0001
+__device__ __forceinline__ float clamp_edge(float v, float below) {
+    if (v < below) return 0.0001f;
+    if (v > 1.f) return 1.f;
     return v;
 }
 
-// DistanceTriangle (bvh.cpp:212-242)
-__device__ float distance_triangle(v3 p, v3 a, v3 b, v3 c) {
-    const v3 ba = vsub(b, a), pa = vsub(p, a);
-    const v3 cb = vsub(c, b), pb = vsub(p, b);
-    const v3 ac = vsub(a, c), pc = vsub(p, c);
-    const v3 nor = cross_d(ba, ac);
-    const float s = fa(fa(sgn(vdot(cross_d(ba, nor), pa)), sgn(vdot(cross_d(cb, nor), pb))),
-                       sgn(vdot(cross_d(ac, nor), pc)));
-    float q;
-    if ((double)s < 2.0) {
-        const float e0 = vlen2(vsub(vmul(ba, clamp_edge(fdv(vdot(ba, pa), vlen2(ba)))), pa));
-        const float e1 = vlen2(vsub(vmul(cb, clamp_edge(fdv(vdot(cb, pb), vlen2(cb)))), pb));
-        const float e2 = vlen2(vsub(vmul(ac, clamp_edge(fdv(vdot(ac, pc), vlen2(ac)))), pc));
-        q = rmin(rmin(e0, e1), e2);
-    } else {
-        const float d = vdot(nor, pa);
-        q = fdv(fm(d, d), vlen2(nor));
+// What DistanceTriangle (bvh.cpp:212-242) takes from the triangle alone, in 9 float4
+struct TriDist {
+    v3 a, b, c, ba, cb, ac, nor, n0, n1, n2;   // n0 = Cross(ba, nor) and so on
+    float l0, l1, l2, ln;                      // |ba|^2, |cb|^2, |ac|^2, |nor|^2
+};
+constexpr int kDistRec = 36, kRayRec = 12;   // floats per triangle (34 and 9 used)
+
+__device__ __forceinline__ TriDist load_dist(const float4 *__restrict__ r) {
+    const float4 q0 = __ldg(r), q1 = __ldg(r + 1), q2 = __ldg(r + 2), q3 = __ldg(r + 3), q4 = __ldg(r + 4);
+    const float4 q5 = __ldg(r + 5), q6 = __ldg(r + 6), q7 = __ldg(r + 7), q8 = __ldg(r + 8);
+    TriDist t;
+    t.a = V(q0.x, q0.y, q0.z); t.b = V(q0.w, q1.x, q1.y); t.c = V(q1.z, q1.w, q2.x);
+    t.ba = V(q2.y, q2.z, q2.w); t.cb = V(q3.x, q3.y, q3.z); t.ac = V(q3.w, q4.x, q4.y);
+    t.nor = V(q4.z, q4.w, q5.x); t.n0 = V(q5.y, q5.z, q5.w); t.n1 = V(q6.x, q6.y, q6.z);
+    t.n2 = V(q6.w, q7.x, q7.y);
+    t.l0 = q7.z; t.l1 = q7.w; t.l2 = q8.x; t.ln = q8.y;
+    return t;
+}
+
+// The squared DistanceTriangle: the reference's value is its square root, which keeps order, so
+// the least one is rooted once.
+__device__ __forceinline__ float distance_triangle2(v3 p, const TriDist &t, float below) {
+    const v3 pa = vsub(p, t.a), pb = vsub(p, t.b), pc = vsub(p, t.c);
+    const float s = fa(fa(sgn(vdot(t.n0, pa)), sgn(vdot(t.n1, pb))), sgn(vdot(t.n2, pc)));
+    if (s < 2.f) {
+        const float e0 = vlen2(vsub(vmul(t.ba, clamp_edge(fdv(vdot(t.ba, pa), t.l0), below)), pa));
+        const float e1 = vlen2(vsub(vmul(t.cb, clamp_edge(fdv(vdot(t.cb, pb), t.l1), below)), pb));
+        const float e2 = vlen2(vsub(vmul(t.ac, clamp_edge(fdv(vdot(t.ac, pc), t.l2), below)), pc));
+        return rmin(rmin(e0, e1), e2);
     }
-    return __fsqrt_rn(q);
+    const float d = vdot(t.nor, pa);
+    return fdv(fm(d, d), t.ln);
+}
+
+// The records of every triangle: corners for the ray passes (the caller's order), TriDist for
+// the distance pass (the Morton-ordered copy).
+__global__ void k_mesh_records(const float *__restrict__ tri, const float *__restrict__ dtri, int ntri,
+                               float *__restrict__ ray, float *__restrict__ dist) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ntri) return;
+    for (int k = 0; k < 9; k++) ray[kRayRec * (size_t)t + k] = tri[9 * (size_t)t + k];
+    const float *q = dtri + 9 * (size_t)t;
+    const v3 a = V(q[0], q[1], q[2]), b = V(q[3], q[4], q[5]), c = V(q[6], q[7], q[8]);
+    const v3 ba = vsub(b, a), cb = vsub(c, b), ac = vsub(a, c);
+    const v3 nor = cross_d(ba, ac);
+    const v3 v[10] = {a, b, c, ba, cb, ac, nor, cross_d(ba, nor), cross_d(cb, nor), cross_d(ac, nor)};
+    float *o = dist + kDistRec * (size_t)t;
+    for (int k = 0; k < 10; k++) {
+        o[3 * k] = v[k].x;
+        o[3 * k + 1] = v[k].y;
+        o[3 * k + 2] = v[k].z;
+    }
+    o[30] = vlen2(ba);
+    o[31] = vlen2(cb);
+    o[32] = vlen2(ac);
+    o[33] = vlen2(nor);
+    o[34] = o[35] = 0.f;
 }
 
 __device__ __forceinline__ float comp(v3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
@@ -73,27 +111,41 @@ __device__ __forceinline__ v3 permute(v3 v, int x, int y, int z) { return V(comp
 __device__ __forceinline__ float max3abs(float a, float b, float c) {   // MaxComponent(Abs(v))
     return rmax(fabsf(a), rmax(fabsf(b), fabsf(c)));
 }
-__device__ __forceinline__ bool is_zero(float a) { return (double)fabsf(a) < 1e-8; }
 
-struct Gammas { float g2, g3, g5, g7; };
+// error-bound factors, and the least floats not below 1e-8 and 0.0001 (double comparisons)
+struct Gammas { float g2, g3, g5, g7, zero, edge; };
+
+// A direction with what IntersectTriangle and Bounds3::Intersect take from it alone
+struct RayDir {
+    v3 dir, inv;          // 1 / dir
+    float sx, sy, sz;     // shear to the frame whose z is dir's largest axis
+    int kx, ky, kz;
+};
+__device__ __forceinline__ RayDir ray_dir(v3 dir) {
+    RayDir r;
+    r.dir = dir;
+    r.inv = V(fdv(1.f, dir.x), fdv(1.f, dir.y), fdv(1.f, dir.z));
+    const v3 ad = V(fabsf(dir.x), fabsf(dir.y), fabsf(dir.z));
+    r.kz = (ad.x > ad.y) ? ((ad.x > ad.z) ? 0 : 2) : ((ad.y > ad.z) ? 1 : 2);
+    r.kx = r.kz == 2 ? 0 : r.kz + 1;
+    r.ky = r.kx == 2 ? 0 : r.kx + 1;
+    const v3 d = permute(dir, r.kx, r.ky, r.kz);
+    r.sx = fdv(-d.x, d.z);
+    r.sy = fdv(-d.y, d.z);
+    r.sz = fdv(1.f, d.z);
+    return r;
+}
 
 struct Hit { v3 p, err, n; float t; };
 
 // IntersectTriangle (bvh.cpp:244-373) against a ray with tMax; on a hit, tmax and hit
 // are updated.
-__device__ bool intersect_triangle(v3 o, v3 dir, float &tmax, v3 p0, v3 p1, v3 p2, const Gammas &G, Hit &hit) {
-    v3 p0t = vsub(p0, o), p1t = vsub(p1, o), p2t = vsub(p2, o);
-    const v3 ad = V(fabsf(dir.x), fabsf(dir.y), fabsf(dir.z));
-    const int kz = (ad.x > ad.y) ? ((ad.x > ad.z) ? 0 : 2) : ((ad.y > ad.z) ? 1 : 2);
-    int kx = kz + 1;
-    if (kx == 3) kx = 0;
-    int ky = kx + 1;
-    if (ky == 3) ky = 0;
-    const v3 d = permute(dir, kx, ky, kz);
-    p0t = permute(p0t, kx, ky, kz);
-    p1t = permute(p1t, kx, ky, kz);
-    p2t = permute(p2t, kx, ky, kz);
-    const float sx = fdv(-d.x, d.z), sy = fdv(-d.y, d.z), sz = fdv(1.f, d.z);
+__device__ __forceinline__ bool intersect_triangle(v3 o, const RayDir &R, float &tmax, v3 p0, v3 p1, v3 p2,
+                                                   const Gammas &G, Hit &hit) {
+    const float sx = R.sx, sy = R.sy, sz = R.sz;
+    v3 p0t = permute(vsub(p0, o), R.kx, R.ky, R.kz);
+    v3 p1t = permute(vsub(p1, o), R.kx, R.ky, R.kz);
+    v3 p2t = permute(vsub(p2, o), R.kx, R.ky, R.kz);
     p0t.x = fa(p0t.x, fm(sx, p0t.z));
     p0t.y = fa(p0t.y, fm(sy, p0t.z));
     p1t.x = fa(p1t.x, fm(sx, p1t.z));
@@ -103,14 +155,14 @@ __device__ bool intersect_triangle(v3 o, v3 dir, float &tmax, v3 p0, v3 p1, v3 p
     float e0 = fs(fm(p1t.x, p2t.y), fm(p1t.y, p2t.x));
     float e1 = fs(fm(p2t.x, p0t.y), fm(p2t.y, p0t.x));
     float e2 = fs(fm(p0t.x, p1t.y), fm(p0t.y, p1t.x));
-    if (is_zero(e0) || is_zero(e1) || is_zero(e2)) {
+    if (fabsf(e0) < G.zero || fabsf(e1) < G.zero || fabsf(e2) < G.zero) {
         e0 = __double2float_rn(__dsub_rn(__dmul_rn((double)p2t.y, (double)p1t.x), __dmul_rn((double)p2t.x, (double)p1t.y)));
         e1 = __double2float_rn(__dsub_rn(__dmul_rn((double)p0t.y, (double)p2t.x), __dmul_rn((double)p0t.x, (double)p2t.y)));
         e2 = __double2float_rn(__dsub_rn(__dmul_rn((double)p1t.y, (double)p0t.x), __dmul_rn((double)p1t.x, (double)p0t.y)));
     }
     if ((e0 < 0.f || e1 < 0.f || e2 < 0.f) && (e0 > 0.f || e1 > 0.f || e2 > 0.f)) return false;
     const float det = fa(fa(e0, e1), e2);
-    if (is_zero(det)) return false;
+    if (fabsf(det) < G.zero) return false;
     p0t.z = fm(p0t.z, sz);
     p1t.z = fm(p1t.z, sz);
     p2t.z = fm(p2t.z, sz);
@@ -142,14 +194,14 @@ __device__ bool intersect_triangle(v3 o, v3 dir, float &tmax, v3 p0, v3 p1, v3 p
     return true;
 }
 
-// Bounds3::Intersect of the mesh bounds (geometry.h:1881-1898)
-__device__ bool hits_bounds(v3 lo, v3 hi, v3 o, v3 d, float tmax, float g3) {
+// Bounds3::Intersect (geometry.h:1881-1898)
+__device__ __forceinline__ bool hits_bounds(v3 lo, v3 hi, v3 o, v3 inv, float tmax, float g3) {
     float t0 = 0.f, t1 = tmax;
     const float grow = fa(1.f, fm(2.f, g3));
+#pragma unroll
     for (int k = 0; k < 3; k++) {
-        const float inv = fdv(1.f, comp(d, k));
-        float tn = fm(fs(comp(lo, k), comp(o, k)), inv);
-        float tf = fm(fs(comp(hi, k), comp(o, k)), inv);
+        float tn = fm(fs(comp(lo, k), comp(o, k)), comp(inv, k));
+        float tf = fm(fs(comp(hi, k), comp(o, k)), comp(inv, k));
         if (tn > tf) {
             const float x = tn;
             tn = tf;
@@ -206,38 +258,41 @@ constexpr int kMaxRayHits = 256;   // a ray stuck on degenerate geometry gives u
 constexpr int kMeshTile = 64;
 constexpr int kMeshSub = 8;
 
-// The box tests of the two passes.
-__device__ __forceinline__ bool box_near(const float *__restrict__ bx, v3 p, float d, float margin) {
-    const float ex = fmaxf(fmaxf(__ldg(&bx[0]) - p.x, p.x - __ldg(&bx[3])), 0.f);
-    const float ey = fmaxf(fmaxf(__ldg(&bx[1]) - p.y, p.y - __ldg(&bx[4])), 0.f);
-    const float ez = fmaxf(fmaxf(__ldg(&bx[2]) - p.z, p.z - __ldg(&bx[5])), 0.f);
-    return !(sqrtf(ex * ex + ey * ey + ez * ez) > d * 1.01f + margin);
+// Boxes: 8 floats each, low corner then high corner.  Squared distance of p to a box:
+__device__ __forceinline__ float box_distance2(const float4 *__restrict__ bx, v3 p) {
+    const float4 l = __ldg(bx), h = __ldg(bx + 1);
+    const float ex = fmaxf(fmaxf(l.x - p.x, p.x - h.x), 0.f);
+    const float ey = fmaxf(fmaxf(l.y - p.y, p.y - h.y), 0.f);
+    const float ez = fmaxf(fmaxf(l.z - p.z, p.z - h.z), 0.f);
+    return ex * ex + ey * ey + ez * ez;
 }
 
-__device__ __forceinline__ bool box_on_ray(const float *__restrict__ bx, v3 o, v3 dir, float tmax, float g3) {
-    return hits_bounds(V(__ldg(&bx[0]), __ldg(&bx[1]), __ldg(&bx[2])), V(__ldg(&bx[3]), __ldg(&bx[4]), __ldg(&bx[5])), o,
-                       dir, tmax, g3);
+__device__ __forceinline__ bool box_on_ray(const float4 *__restrict__ bx, v3 o, v3 inv, float tmax, float g3) {
+    const float4 l = __ldg(bx), h = __ldg(bx + 1);
+    return hits_bounds(V(l.x, l.y, l.z), V(h.x, h.y, h.z), o, inv, tmax, g3);
 }
 
 // f(t) for every triangle t of the tiles and sub-tiles that keep(box) accepts, in order
 template <class Keep, class F>
-__device__ __forceinline__ void mesh_walk(const float *__restrict__ tiles, int ntri, Keep &&keep, F &&f) {
+__device__ __forceinline__ void mesh_walk(const float4 *__restrict__ tiles, int ntri, Keep &&keep, F &&f) {
     const int ntiles = (ntri + kMeshTile - 1) / kMeshTile, nsub = (ntri + kMeshSub - 1) / kMeshSub;
-    const float *sub = tiles + 6 * ntiles;
+    const float4 *sub = tiles + 2 * ntiles;
     for (int b = 0; b < ntiles; b++) {
-        if (!keep(tiles + 6 * b)) continue;
+        if (!keep(tiles + 2 * b)) continue;
         const int s1 = min(nsub, (b + 1) * (kMeshTile / kMeshSub));
         for (int q = b * (kMeshTile / kMeshSub); q < s1; q++) {
-            if (!keep(sub + 6 * q)) continue;
+            if (!keep(sub + 2 * q)) continue;
             const int t1 = min(ntri, (q + 1) * kMeshSub);
             for (int t = q * kMeshSub; t < t1; t++) f(t);
         }
     }
 }
 
-__global__ void k_mesh_sdf(const float *__restrict__ tri, int ntri, const float *__restrict__ tiles,
-                           const float *__restrict__ dtri, const float *__restrict__ dtiles, float margin,
-                           SdfDev g, v3 lo, v3 hi, Gammas G, float *__restrict__ out, unsigned *__restrict__ stuck) {
+// Bound: FP32 issue slots of the triangle tests (boxes cull all but about a tenth of them).
+__global__ void __launch_bounds__(128)
+k_mesh_sdf(const float4 *__restrict__ ray, int ntri, const float4 *__restrict__ tiles, const float4 *__restrict__ dist,
+           const float4 *__restrict__ dtiles, float margin, SdfDev g, v3 lo, v3 hi, Gammas G, float *__restrict__ out,
+           unsigned *__restrict__ stuck) {
     const unsigned total = (unsigned)g.nx * (unsigned)g.ny * (unsigned)g.nz;
     const unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= total) return;
@@ -247,16 +302,49 @@ __global__ void k_mesh_sdf(const float *__restrict__ tri, int ntri, const float 
     const v3 p = V(fa(g.org[0], fm(g.sp[0], (float)i)), fa(g.org[1], fm(g.sp[1], (float)j)),
                    fa(g.org[2], fm(g.sp[2], (float)k)));
     // MeshClosestDistance: the least DistanceTriangle (strictly smaller replaces; the least
-    // value does not depend on the order, so this pass walks the Morton-ordered copy)
+    // value does not depend on the order, so this pass walks the Morton-ordered copy, the
+    // sub-tile whose box is nearest first: its distances leave little of the rest)
     float d = 3.1622776601683794e+18f;   // SqrtInfinity
-    mesh_walk(dtiles, ntri, [&](const float *bx) { return box_near(bx, p, d, margin); }, [&](int t) {
-        const float dt = distance_triangle(p, tri_vertex(dtri, t, 0), tri_vertex(dtri, t, 1), tri_vertex(dtri, t, 2));
-        if (dt < d) d = dt;
-    });
+    float q2 = __int_as_float(0x7f800000), reach2 = q2;   // least squared distance, and of a box that matters
+    auto visit = [&](int t) {
+        const float q = distance_triangle2(p, load_dist(dist + (kDistRec / 4) * (size_t)t), G.edge);
+        if (q < q2) {
+            q2 = q;
+            const float r = sqrtf(q) * 1.01f + margin;
+            reach2 = r * r * 1.0001f;
+        }
+    };
+    {
+        const int ntiles = (ntri + kMeshTile - 1) / kMeshTile, nsub = (ntri + kMeshSub - 1) / kMeshSub;
+        const float4 *sub = dtiles + 2 * ntiles;
+        int tile = 0, first = 0;
+        float near2 = box_distance2(dtiles, p);
+        for (int b = 1; b < ntiles; b++) {
+            const float e = box_distance2(dtiles + 2 * b, p);
+            if (e < near2) {
+                near2 = e;
+                tile = b;
+            }
+        }
+        first = tile * (kMeshTile / kMeshSub);
+        const int s1 = min(nsub, first + kMeshTile / kMeshSub);
+        near2 = box_distance2(sub + 2 * first, p);
+        for (int b = first + 1; b < s1; b++) {
+            const float e = box_distance2(sub + 2 * b, p);
+            if (e < near2) {
+                near2 = e;
+                first = b;
+            }
+        }
+        for (int t = first * kMeshSub; t < min(ntri, (first + 1) * kMeshSub); t++) visit(t);
+    }
+    mesh_walk(dtiles, ntri, [&](const float4 *bx) { return !(box_distance2(bx, p) > reach2); }, visit);
+    const float root = __fsqrt_rn(q2);
+    if (root < d) d = root;
     // MeshIsPointInside: ray towards the bounds' centre, closest hits counted
     const v3 center = vmul(vadd(lo, hi), 0.5f);
     const v3 to = vsub(center, p);
-    const v3 dir = vdiv(to, vlen(to));
+    const RayDir R = ray_dir(vdiv(to, vlen(to)));
     v3 o = p;
     int hits = 0;
     bool done = false;
@@ -264,17 +352,18 @@ __global__ void k_mesh_sdf(const float *__restrict__ tri, int ntri, const float 
         float tmax = 3.402823466e+38f;   // Infinity
         Hit h;
         bool any = false;
-        if (hits_bounds(lo, hi, o, dir, tmax, G.g3)) {
-            mesh_walk(tiles, ntri, [&](const float *bx) { return box_on_ray(bx, o, dir, tmax, G.g3); }, [&](int t) {
-                any |= intersect_triangle(o, dir, tmax, tri_vertex(tri, t, 0), tri_vertex(tri, t, 1),
-                                          tri_vertex(tri, t, 2), G, h);
+        if (hits_bounds(lo, hi, o, R.inv, tmax, G.g3)) {
+            mesh_walk(tiles, ntri, [&](const float4 *bx) { return box_on_ray(bx, o, R.inv, tmax, G.g3); }, [&](int t) {
+                const float4 *q = ray + (kRayRec / 4) * (size_t)t;
+                const float4 u = __ldg(q), v = __ldg(q + 1), w = __ldg(q + 2);
+                any |= intersect_triangle(o, R, tmax, V(u.x, u.y, u.z), V(u.w, v.x, v.y), V(v.z, v.w, w.x), G, h);
             });
         }
         if (!any) {
             done = true;
         } else {
             hits++;
-            o = offset_origin(h, dir);
+            o = offset_origin(h, R.dir);
         }
     }
     if (!done) {
@@ -288,29 +377,30 @@ __global__ void k_mesh_sdf(const float *__restrict__ tri, int ntri, const float 
 
 }  // namespace
 
-// boxes of the tiles, then of the sub-tiles (6 floats each)
+// boxes of the tiles, then of the sub-tiles (8 floats each)
 int mesh_tiles(int ntri) { return (ntri + kMeshTile - 1) / kMeshTile + (ntri + kMeshSub - 1) / kMeshSub; }
 
 static void tile_boxes(const float *tri, int ntri, int size, float *tiles) {
     for (int b = 0; b < (ntri + size - 1) / size; b++) {
-        float *bx = tiles + 6 * b;
+        float *bx = tiles + 8 * b;
         for (int k = 0; k < 3; k++) {
             bx[k] = 3.402823466e+38f;
-            bx[3 + k] = -3.402823466e+38f;
+            bx[4 + k] = -3.402823466e+38f;
         }
+        bx[3] = bx[7] = 0.f;
         for (int t = b * size; t < ntri && t < (b + 1) * size; t++)
             for (int c = 0; c < 3; c++)
                 for (int k = 0; k < 3; k++) {
                     const float x = tri[9 * (size_t)t + 3 * c + k];
                     bx[k] = x < bx[k] ? x : bx[k];
-                    bx[3 + k] = x > bx[3 + k] ? x : bx[3 + k];
+                    bx[4 + k] = x > bx[4 + k] ? x : bx[4 + k];
                 }
     }
 }
 
 void mesh_tile_bounds(const float *tri, int ntri, float *tiles) {
     tile_boxes(tri, ntri, kMeshTile, tiles);
-    tile_boxes(tri, ntri, kMeshSub, tiles + 6 * ((ntri + kMeshTile - 1) / kMeshTile));
+    tile_boxes(tri, ntri, kMeshSub, tiles + 8 * ((ntri + kMeshTile - 1) / kMeshTile));
 }
 
 // The triangles in the Morton order of their centroids (30-bit codes in the mesh bounds,
@@ -336,19 +426,21 @@ void mesh_morton_order(const float *tri, int ntri, const float lo[3], const floa
         for (int q = 0; q < 9; q++) sorted[9 * (size_t)r + q] = tri[9 * (size_t)key[(size_t)r].second + q];
 }
 
+size_t mesh_record_floats(int ntri) { return (size_t)(kDistRec + kRayRec) * (size_t)ntri; }
+
 void launch_mesh_sdf(const float *tri, int ntri, const float *tiles, const float *dtri, const float *dtiles,
                      float margin, const SdfDev &g, const float lo[3], const float hi[3], const float gamma[4],
-                     float *out, unsigned *stuck, cudaStream_t s) {
+                     const float least[2], float *records, float *out, unsigned *stuck, cudaStream_t s) {
     const long long total = (long long)g.nx * g.ny * g.nz;
-    Gammas G;
-    G.g2 = gamma[0];
-    G.g3 = gamma[1];
-    G.g5 = gamma[2];
-    G.g7 = gamma[3];
+    const Gammas G = {gamma[0], gamma[1], gamma[2], gamma[3], least[0], least[1]};
     v3 l, h;
     l.x = lo[0]; l.y = lo[1]; l.z = lo[2];
     h.x = hi[0]; h.y = hi[1]; h.z = hi[2];
-    k_mesh_sdf<<<blocks_for(total, 128), 128, 0, s>>>(tri, ntri, tiles, dtri, dtiles, margin, g, l, h, G, out, stuck);
+    float *dist = records, *ray = records + (size_t)kDistRec * (size_t)ntri;
+    k_mesh_records<<<blocks_for(ntri, 128), 128, 0, s>>>(tri, dtri, ntri, ray, dist);
+    const auto quads = [](const float *p) { return reinterpret_cast<const float4 *>(p); };
+    k_mesh_sdf<<<blocks_for(total, 128), 128, 0, s>>>(quads(ray), ntri, quads(tiles), quads(dist), quads(dtiles), margin,
+                                                      g, l, h, G, out, stuck);
 }
 
 }  // namespace bbg

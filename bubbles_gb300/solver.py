@@ -213,7 +213,7 @@ class Solver:
         cnt = ctypes.c_size_t()
         stuck = ctypes.c_int()
         args = (self.h, v.ctypes.data, len(v), t.ctypes.data, len(t), float(dx), float(margin), ctypes.byref(g))
-        N.call("bbg_mesh_sdf", *args, None, 0, ctypes.byref(cnt), ctypes.byref(stuck))
+        N.call("bbg_mesh_sdf", *args, None, 0, ctypes.byref(cnt), None)   # the size: nothing is computed
         vals = np.empty(cnt.value, np.float32)
         N.call("bbg_mesh_sdf", *args, vals.ctypes.data, vals.size, ctypes.byref(cnt), ctypes.byref(stuck))
         return (np.array(g.nodes[:]), np.array(g.origin[:]), np.array(g.spacing[:]), vals,
