@@ -366,6 +366,16 @@ static bbg_status lnm_finish(bbg_solver s, cudaError_t e, const LnmScratch &w, i
     return BBG_OK;
 }
 
+// The largest float x with sqrtf(x) <= bound (sqrtf keeps order, so x <= it decides the same);
+// -1 for a bound below 0, which no distance meets.
+static float largest_square(float bound) {
+    if (!(bound >= 0.f)) return -1.f;
+    float x = bound * bound;
+    while (std::sqrt(x) > bound) x = std::nextafterf(x, -1.f);
+    while (std::isfinite(x) && std::sqrt(std::nextafterf(x, HUGE_VALF)) <= bound) x = std::nextafterf(x, HUGE_VALF);
+    return x;
+}
+
 // The particle tests' arguments: Xiaowei at kernel radius 6h (xiaowei.h:26-33), Dilts at
 // 0.75 x the set's radius (the target spacing, particle.h:536-541; dilts.h:30-33), the
 // spoke angles i pi / 64 and j 2 pi / 64 rounded to float and their sines and cosines by
@@ -384,10 +394,13 @@ static BoundaryArgs boundary_args(bbg_solver s, double h) {
     A.x_rhot = (float)(0.7 * 1000.0);
     A.x_h2 = h2;
     A.x_wc = 315.0 / (64.0 * 3.14159265358979323846 * (double)h3);
+    A.x_wh = (float)A.x_wc;
+    A.x_wl = (float)(A.x_wc - (double)A.x_wh);
     A.x_limit = 0.15 * (double)rho6;
     const float radius = (float)s->desc.target_spacing;
     A.d_rad = (float)((double)radius * 0.75);
-    A.d_lim = (A.d_rad + A.d_rad) - 0.0001f;
+    A.d_rad2 = largest_square(A.d_rad);
+    A.d_lim2 = largest_square((A.d_rad + A.d_rad) - 0.0001f);
     const float samples = (float)64;
     for (int i = 0; i <= 64; i++) {
         const float u = (float)(i * 3.14159265358979323846 / (double)samples);
@@ -559,6 +572,8 @@ bbg_status bbg_particle_sdf(bbg_solver s, int method, double kernel_radius, doub
     A.mass = s->mass;
     A.r2 = A.radius * A.radius;
     A.wc = 315.0 / (64.0 * 3.14159265358979323846 * (double)(A.r2 * A.radius));
+    A.wh = (float)A.wc;
+    A.wl = (float)(A.wc - (double)A.wh);
     float *d_out = nullptr;
     cudaError_t e = scratch_begin(s);
     if (e == cudaSuccess) e = scratch_get(s, total, &d_out);

@@ -132,6 +132,55 @@ __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); 
 __device__ __forceinline__ float fs(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fdv(float a, float b) { return __fdiv_rn(a, b); }
 
+// ----------------------------------------------------------------------------
+// Products that the reference takes in double and rounds to float, without FP64 (1/64 of the FP32
+// rate here): the product as an unevaluated sum of two floats (the error of each product by
+// fma, Dekker's double-length arithmetic), relative error below 2^-44, whose rounding to
+// float is that of the reference's double unless the sum lies within 2^-42 of the middle of two
+// floats.  There, and below 2^-70, where the low parts leave the normal range, the double
+// products are done.
+// ----------------------------------------------------------------------------
+struct ff { float h, l; };   // h + l
+
+__device__ __forceinline__ ff ff_mul(ff a, float b) {
+    const float p = fm(a.h, b);
+    return ff{p, __fmaf_rn(a.l, b, __fmaf_rn(a.h, b, -p))};
+}
+// h + l rounded to float; false when the double value may round the other way
+__device__ __forceinline__ bool ff_round(ff a, float *r) {
+    const float up = fa(a.h, __fmaf_rn(a.h, 2.2737368e-13f, a.l));     // 2^-42
+    const float dn = fa(a.h, __fmaf_rn(a.h, -2.2737368e-13f, a.l));
+    *r = up;
+    return up == dn && a.h >= 8.4703295e-22f;                          // 2^-70
+}
+
+// The double products themselves, out of line: inlined, the compiler evaluates them beside the fast
+// path and selects.
+static __device__ __noinline__ float double_cube_exact(double c, double x) {
+    return __double2float_rn(__dmul_rn(__dmul_rn(__dmul_rn(c, x), x), x));
+}
+static __device__ __noinline__ float double_cube_1m_exact(float t2) {
+    const double q = __dsub_rn(1.0, (double)t2);
+    return __double2float_rn(__dmul_rn(__dmul_rn(q, q), q));
+}
+
+// (float)(((wc x) x) x) with every product rounded to double; wh + wl is wc to 48 bits
+__device__ __forceinline__ float double_cube(double wc, float wh, float wl, float x) {
+    float r;
+    if (ff_round(ff_mul(ff_mul(ff_mul(ff{wh, wl}, x), x), x), &r)) return r;
+    return double_cube_exact(wc, (double)x);
+}
+
+// (float)((q q) q), q = 1 - t2 in double, 0 <= t2 <= 1
+__device__ __forceinline__ float double_cube_1m(float t2) {
+    const float h = fs(1.f, t2), l = fs(fs(1.f, h), t2);   // q = h + l exactly
+    const float p = fm(h, h), e = __fmaf_rn(2.f * h, l, __fmaf_rn(h, h, -p));
+    const float p3 = fm(p, h);
+    float r;
+    if (ff_round(ff{p3, __fmaf_rn(e, h, __fmaf_rn(p, l, __fmaf_rn(p, h, -p3)))}, &r)) return r;
+    return double_cube_1m_exact(t2);
+}
+
 struct v3 { float x, y, z; };
 __device__ __forceinline__ v3 V(float x, float y, float z) { v3 r; r.x = x; r.y = y; r.z = z; return r; }
 __device__ __forceinline__ v3 V(float4 a) { return V(a.x, a.y, a.z); }

@@ -148,7 +148,9 @@ struct BoundaryArgs {
     float x_rhot;         // Xiaowei: 0.7 * water density; 6h squared; 315 / (64 pi (6h)^3);
     float x_h2;           // 0.15 * 6h (as double)
     double x_wc, x_limit;
-    float d_rad, d_lim;   // Dilts: 0.75 * radius; 2 rad - Epsilon
+    float x_wh, x_wl;     // x_wc as a sum of two floats
+    float d_rad;          // Dilts: 0.75 * radius; the largest floats whose roots do not pass
+    float d_rad2, d_lim2; // it and 2 rad - Epsilon
     float spoke[260];     // sin u, cos u, sin v, cos v of the 65 spoke angles (host libm)
 };
 void launch_lnm_single(const GridDev &g, const unsigned *start, const unsigned *cell, const int *pid, int n,
@@ -175,6 +177,7 @@ struct SurfaceArgs {
     float offset;         // Zhu-Bridson: radius x threshold
     float mass, r2;       // SPH: particle mass, radius squared,
     double wc;            // 315 / (64 pi radius^3)
+    float wh, wl;         // the same as a sum of two floats
 };
 void launch_particle_sdf(const SurfaceArgs &A, float *out, cudaStream_t s);
 void launch_lnm(const GridDev &g, const unsigned *start, const unsigned *cell, const int *pid, int n, int delta,

@@ -5,7 +5,8 @@
 // the hashed cell and its 27 neighbours in the reference's order (y, then x, then z), each
 // cell's particles in chain order (the slot range of the last distribution).  Every float
 // operation is explicitly rounded in the reference's order; the steps the reference takes
-// in double (the cubic weight of Zhu-Bridson, the std kernel's constant) are double here.
+// in double (the cubic weight of Zhu-Bridson, the std kernel's constant) give the double's result
+// (double_cube): 262,144 particles, 111 -> 70 us.
 #include "bbg_internal.cuh"
 #include "bbg_kernels.h"
 
@@ -50,8 +51,7 @@ __global__ void k_particle_sdf(SurfaceArgs A, float *__restrict__ out) {
                         // ZhuBridsonSDF: k_cub(|p - x| / R) = Max(0, (1 - s^2)^3), the cube in double
                         if (d < R) {
                             const float t = fdv(d, R);
-                            const double q = __dsub_rn(1.0, (double)fm(t, t));
-                            const float cub = __double2float_rn(__dmul_rn(__dmul_rn(q, q), q));
+                            const float cub = double_cube_1m(fm(t, t));
                             const float w = 0.f < cub ? cub : 0.f;
                             wsum = fa(wsum, w);
                             ax = fa(ax, fm(xi.x, w));
@@ -64,8 +64,7 @@ __global__ void k_particle_sdf(SurfaceArgs A, float *__restrict__ out) {
                         const float of = fs(d2, A.r2);
                         float w = 0.f;
                         if (!(fabsf(of) < A.iz || of > 0.f)) {
-                            const double x = (double)fs(1.f, fdv(d2, A.r2));
-                            w = __double2float_rn(__dmul_rn(__dmul_rn(__dmul_rn(A.wc, x), x), x));
+                            w = double_cube(A.wc, A.wh, A.wl, fs(1.f, fdv(d2, A.r2)));
                         }
                         wsum = fa(wsum, fm(fdv(A.mass, A.rho[s]), w));
                     }
