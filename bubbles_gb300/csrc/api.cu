@@ -549,7 +549,7 @@ unsigned fbits(float f) {
 }
 
 // Capture one whole substep (grid rebuild, density, forces, the corrector as a
-// conditional WHILE node driven by k_corrector_control, integration) into a graph.
+// conditional WHILE node ended by its pressure-force pass, integration) into a graph.
 bbg_status capture_substep(bbg_solver s, float dt, int max_it, float delta,
                            bbg_solver_s::SubstepGraph &g) {
     const int st0 = s->state, pid0 = s->pid_cur, work = 1 - st0;
@@ -588,8 +588,7 @@ bbg_status capture_substep(bbg_solver s, float dt, int max_it, float delta,
                                               cudaStreamCaptureModeThreadLocal);
             if (e == cudaSuccess) {
                 launch_pred_density(P, B, work, -1, delta, s->aux, clamp_total(s));
-                launch_pressure_force(P, B, work, -1, max_it, dt, dt / s->mass, s->aux);
-                launch_corrector_control(P, B, max_it, handle, s->aux);
+                launch_pressure_force(P, B, work, -1, max_it, dt, dt / s->mass, s->aux, 0, handle);
                 cudaError_t e2 = cudaStreamEndCapture(s->aux, &body);
                 if (e == cudaSuccess) e = e2;
             }

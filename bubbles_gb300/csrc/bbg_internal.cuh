@@ -112,7 +112,8 @@ struct StepState {
     unsigned nbr_overflow;
     unsigned nonfinite;
     unsigned crowded;                    // cells / particles past the work caps (see below)
-    int iter;                            // corrector iteration (graph-driven loop)
+    int iter, iter_pf;                   // corrector iteration (graph-driven loop): of the predicted-
+                                         // density pass, of the pressure-force pass after it
 };
 
 // Work caps that keep a degenerate state (e.g. a blown-up simulation that piles particles

@@ -99,12 +99,12 @@ void launch_pred_density(const Params &P, const DevBufs &B, int buf, int k, floa
                          cudaStream_t s, int clamp_total = 0);
 // mode 0: pressure force, then the next prediction or (converged) integration;
 // 1: pressure force only; 2: pressure force and prediction, never integration.
+// loop: the conditional node that k < 0 (graph) ends or continues
 void launch_pressure_force(const Params &P, const DevBufs &B, int buf, int k, int max_it,
-                           float dt, float dt_over_m, cudaStream_t s, int mode = 0);
+                           float dt, float dt_over_m, cudaStream_t s, int mode = 0,
+                           cudaGraphConditionalHandle loop = 0);
 // p = scale * previous pressure, rho* = rho, pos.w = p / rho^2
 void launch_warm_start(const Params &P, const DevBufs &B, int buf, float scale, cudaStream_t s);
-void launch_corrector_control(const Params &P, const DevBufs &B, int max_it,
-                              cudaGraphConditionalHandle handle, cudaStream_t s);
 void launch_sph_forces(const Params &P, const DevBufs &B, int buf, float dt, cudaStream_t s);
 void launch_accumulate_integrate(const Params &P, const DevBufs &B, int buf, float dt,
                                  cudaStream_t s);

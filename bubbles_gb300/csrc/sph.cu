@@ -588,11 +588,33 @@ __device__ __forceinline__ void error_reduce(StepState *st, float amax, float as
     }
 }
 
-// k < 0: iteration index from the device counter (the graph's WHILE loop only runs
-// unconverged iterations); k >= 0: host-launched sequence, skip after convergence.
-__device__ __forceinline__ bool corrector_iteration(const Params &P, const StepState *st, int &k) {
+// k < 0: iteration index from the device (the graph's WHILE loop only runs unconverged
+// iterations); k >= 0: host-launched sequence, skip after convergence.  Each pass of the loop
+// advances the other's counter, which no block of its own launch reads: the predicted-density
+// pass hands its iteration to the pressure-force pass, which starts the next one.
+__device__ __forceinline__ bool density_iteration(const Params &P, StepState *st, int &k) {
     if (k < 0) {
         k = st->iter;
+        if (blockIdx.x == 0 && threadIdx.x == 0) st->iter_pf = k;
+        return true;
+    }
+    return !converged_before(P, st, k);
+}
+
+// Also the end of the loop (the break of ComputePressureForceAndIntegrate,
+// pcisph_equations3.cpp:238-246): no further iteration once the density error of iteration k
+// is below tolerance or k was the last allowed one.  The error is final before this launch,
+// so one thread of it decides; a launch of its own for that cost 3 us an iteration.
+__device__ __forceinline__ bool force_iteration(const Params &P, StepState *st, int &k, int max_it,
+                                                cudaGraphConditionalHandle loop) {
+    if (k < 0) {
+        k = st->iter_pf;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            const bool done = (k >= max_it - 1) ||
+                              fdv(__uint_as_float(st->err_bits[k]), P.target_density) < P.max_err_ratio;
+            st->iter = k + 1;
+            cudaGraphSetConditional(loop, done ? 0u : 1u);
+        }
         return true;
     }
     return !converged_before(P, st, k);
@@ -644,7 +666,7 @@ k_pred_density(Params P, float4 *pos, const float4 *__restrict__ xstar,
                const ListEntry *__restrict__ list, const int *__restrict__ nbr, float *__restrict__ press,
                float *__restrict__ rhostar, float *__restrict__ derr, StepState *st, int k,
                float delta, int clamp_total, int wl) {
-    if (!corrector_iteration(P, st, k)) return;
+    if (!density_iteration(P, st, k)) return;
     const int s0 = block_tile(P, wl, PPT * blockDim.x);
     if (s0 < 0 || s0 >= P.n) return;
     float amax = 0.f, asum = 0.f;
@@ -670,7 +692,7 @@ k_pred_density_wl(Params P, float4 *pos, const float4 *__restrict__ xstar,
                   const ListEntry *__restrict__ list, const int *__restrict__ nbr, float *__restrict__ press,
                   float *__restrict__ rhostar, float *__restrict__ derr, StepState *st, int k,
                   float delta, int clamp_total) {
-    if (!corrector_iteration(P, st, k)) return;
+    if (!density_iteration(P, st, k)) return;
     __shared__ int slot[2];
     int parity = 0;
     const int total = worklist_total(P, blockDim.x);
@@ -764,8 +786,8 @@ k_pressure_force(Params P, const float4 *__restrict__ pos, const float4 *__restr
                  float4 *__restrict__ pforce,
                  float4 *__restrict__ xstar, float4 *__restrict__ pos_out,
                  float4 *__restrict__ vel_out, StepState *st, int k, int max_it, float dt,
-                 float dt_over_m, int mode, int wl) {
-    if (!corrector_iteration(P, st, k)) return;
+                 float dt_over_m, int mode, int wl, cudaGraphConditionalHandle loop) {
+    if (!force_iteration(P, st, k, max_it, loop)) return;
     const bool last = corrector_ends(P, st, k, max_it, mode);
     const int s0 = block_tile(P, wl, PPT * blockDim.x);
     if (s0 < 0 || s0 >= P.n) return;
@@ -790,8 +812,8 @@ k_pressure_force_wl(Params P, const float4 *__restrict__ pos, const float4 *__re
                     const ListEntry *__restrict__ list, const int *__restrict__ nbr, float4 *__restrict__ force,
                     float4 *__restrict__ pforce, float4 *__restrict__ xstar, float4 *__restrict__ pos_out,
                     float4 *__restrict__ vel_out, StepState *st, int k, int max_it, float dt, float dt_over_m,
-                    int mode) {
-    if (!corrector_iteration(P, st, k)) return;
+                    int mode, cudaGraphConditionalHandle loop) {
+    if (!force_iteration(P, st, k, max_it, loop)) return;
     __shared__ int slot[2];
     int parity = 0;
     const int total = worklist_total(P, blockDim.x);
@@ -892,18 +914,6 @@ k_worklist(Params P, const StepState *st, int k, int tile) {
         P.wl_ctr[0] = 0;
         P.wl_ctr[1] = 0;
     }
-}
-
-// End of one corrector iteration in the graph-driven loop: stop when the density error
-// of iteration k is below tolerance or k was the last allowed iteration (the break of
-// ComputePressureForceAndIntegrate, pcisph_equations3.cpp:238-246).
-__global__ void k_corrector_control(Params P, StepState *st, int max_it,
-                                    cudaGraphConditionalHandle handle) {
-    const int k = st->iter;
-    const bool done = (k >= max_it - 1) ||
-                      fdv(__uint_as_float(st->err_bits[k]), P.target_density) < P.max_err_ratio;
-    st->iter = k + 1;
-    cudaGraphSetConditional(handle, done ? 0u : 1u);
 }
 
 // ComputeAllForcesFor (sph_equations3.cpp:184-278, extended = 0) in Jacobi order: the
@@ -1225,7 +1235,7 @@ void launch_pack_acoef(const Params &P, const DevBufs &B, int buf, cudaStream_t 
 }
 
 void launch_pressure_force(const Params &P, const DevBufs &B, int buf, int k, int max_it, float dt,
-                           float dt_over_m, cudaStream_t s, int mode) {
+                           float dt_over_m, cudaStream_t s, int mode, cudaGraphConditionalHandle loop) {
     BBG_PBEGIN(B, KID_PRESSURE_FORCE, s, k);
     const int t = B.tune.block;
     const int wl = P.nscenes > 0 ? B.tune.worklist : 0;
@@ -1236,7 +1246,7 @@ void launch_pressure_force(const Params &P, const DevBufs &B, int buf, int k, in
 #define PF_LAUNCH(NB)                                                                                   \
     k_pressure_force_wl<NB><<<B.tune.wl_grid_pf > 0 ? B.tune.wl_grid_pf : pf_grid<NB>(t), t, 0, s>>>(    \
         P, B.pos[buf], B.vel[buf], B.cell, B.start, B.list, B.nbr, B.force, B.pforce, B.xstar,           \
-        B.pos[1 - buf], B.vel[1 - buf], B.st, k, max_it, dt, dt_over_m, mode)
+        B.pos[1 - buf], B.vel[1 - buf], B.st, k, max_it, dt, dt_over_m, mode, loop)
         switch (B.tune.batch_pf) {
             case 2: PF_LAUNCH(2); break;
             case 8: PF_LAUNCH(8); break;
@@ -1251,7 +1261,7 @@ void launch_pressure_force(const Params &P, const DevBufs &B, int buf, int k, in
 #define PF_LAUNCH(NB, PPT)                                                                             \
     k_pressure_force<NB, PPT><<<grid, t, 0, s>>>(                                                       \
         Q, B.pos[buf], B.vel[buf], B.cell, B.start, B.list, B.nbr, B.force, B.pforce, B.xstar,           \
-        B.pos[1 - buf], B.vel[1 - buf], B.st, k, max_it, dt, dt_over_m, mode, wl)
+        B.pos[1 - buf], B.vel[1 - buf], B.st, k, max_it, dt, dt_over_m, mode, wl, loop)
         switch (B.tune.batch_pf * 10 + ppt) {
             case 21: PF_LAUNCH(2, 1); break;
             case 81: PF_LAUNCH(8, 1); break;
@@ -1263,11 +1273,6 @@ void launch_pressure_force(const Params &P, const DevBufs &B, int buf, int k, in
 #undef PF_LAUNCH
     }
     BBG_PEND(B, s);
-}
-
-void launch_corrector_control(const Params &P, const DevBufs &B, int max_it,
-                              cudaGraphConditionalHandle handle, cudaStream_t s) {
-    k_corrector_control<<<1, 1, 0, s>>>(P, B.st, max_it, handle);
 }
 
 void launch_sph_forces(const Params &P, const DevBufs &B, int buf, float dt, cudaStream_t s) {
