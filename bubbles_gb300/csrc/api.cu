@@ -563,10 +563,10 @@ bbg_status capture_substep(bbg_solver s, float dt, int max_it, float delta,
         e = cudaMemsetAsync(s->d_sst, 0, sizeof(SceneState) * (size_t)s->nscenes, cs);
     launch_grid_update(P, B, st0, pid0, cs, s->mlp.divsum, s->mlp.divprev);
     if (s->desc.solver_kind == BBG_SOLVER_SPH) {
-        launch_density(P, B, work, 1, cs);
+        launch_density(P, B, work, 1, cs, true);
         launch_sph_forces(P, B, work, dt, cs);
     } else {
-        launch_density(P, B, work, 0, cs);
+        launch_density(P, B, work, 0, cs, true);
         launch_prologue(s, work, dt, delta, max_it, cs);
         cudaStreamCaptureStatus status;
         cudaGraph_t cg = nullptr;
@@ -682,7 +682,7 @@ bbg_status substep(bbg_solver s, float dt) {
     bbg_status r = grid_update(s);
     if (r) return r;
     if (s->desc.solver_kind == BBG_SOLVER_SPH) {
-        launch_density(s->P, s->B, s->state, 1, s->stream);
+        launch_density(s->P, s->B, s->state, 1, s->stream, true);
         launch_sph_forces(s->P, s->B, s->state, dt, s->stream);
         CK_LAUNCH();
         s->list_state = s->state;
@@ -690,7 +690,7 @@ bbg_status substep(bbg_solver s, float dt) {
         s->valid |= kPosVel | bit(BBG_FIELD_DENSITY) | bit(BBG_FIELD_PRESSURE) | bit(BBG_FIELD_FORCE);
         return pseudo_viscosity(s, dt);
     }
-    launch_density(s->P, s->B, s->state, 0, s->stream);
+    launch_density(s->P, s->B, s->state, 0, s->stream, true);
     launch_prologue(s, s->state, dt, delta, max_it, s->stream);
     CK_LAUNCH();
     s->list_state = s->state;

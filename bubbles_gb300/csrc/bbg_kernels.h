@@ -78,8 +78,9 @@ void launch_fill_vec(float4 *dst, float x, float y, float z, int n, cudaStream_t
 void launch_max_force(const float4 *force, int n, unsigned *out_bits, cudaStream_t s);
 
 // sph.cu
+// recorded: the positions of buf are those of the last grid update, which wrote the filter's records
 void launch_density(const Params &P, const DevBufs &B, int buf, int compute_pressure,
-                    cudaStream_t s);
+                    cudaStream_t s, bool recorded = false);
 // members (other than itself, as original ids) of every particle with original id in
 // [a, b) at the last density pass on buffer buf: counts[id - a], maxm ids per row of out
 void launch_export_members(const Params &P, const DevBufs &B, int buf, int pid_buf, int a, int b, int maxm,

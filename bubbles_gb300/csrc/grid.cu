@@ -4,8 +4,7 @@
 // (src/core/grid.h:391-494, src/equations/sph_equations3.cpp:487-539) with a full
 // counting sort every substep:
 //   1. hash + count:  cell id of every particle (exact reference hash) and its arrival
-//                     index inside the cell, one atomic per distinct cell per warp
-//                     (__match_any_sync aggregation);
+//                     index inside the cell, one atomic per run of equal cells in a warp;
 //   2. scan:          exclusive scan of the per-cell counts -> cell start offsets (tile
 //                     totals, then each tile's scan plus the sum of the tiles before it);
 //   3. place:         (original id, old slot) written into its cell's range;
@@ -14,7 +13,8 @@
 //                     stable sort by (cell id, particle index) -- the reference's chain
 //                     order right after DistributeByParticle (grid.h:391-407) --
 //                     independent of atomic arrival order; position, velocity and id
-//                     are gathered into the other ping-pong buffer.
+//                     are gathered into the other ping-pong buffer, and the density pass's
+//                     filter records written.
 // The reference's incremental update (DistributeToCellOpt) yields the same cell
 // contents; only the chain order differs, which changes FP32 sum order, not sets.
 #include "bbg_kernels.h"
@@ -28,6 +28,9 @@ constexpr int kScanTile = kScanThreads * kScanItems;
 
 static inline int blocks_for(long long n, int t) { return (int)((n + t - 1) / t); }
 
+// (Also adding up the scan tiles' totals here, to save k_scan_reduce's launch, was slower: the few
+// hundred totals take one atomic a warp or more, 20 -> 36 us at 1M particles, and four particles
+// a thread 48 us.)
 __global__ void __launch_bounds__(kThreads)
 k_hash_count(Params P, const float4 *__restrict__ pos, int n, unsigned *__restrict__ cell_old,
              unsigned *__restrict__ sub, unsigned *__restrict__ count, StepState *st) {
@@ -35,15 +38,21 @@ k_hash_count(Params P, const float4 *__restrict__ pos, int n, unsigned *__restri
     const bool valid = i < n;
     unsigned bad = 0, c = 0xffffffffu;
     if (valid) c = grid_hash(P.g, pos[i], P.iz, &bad);
-    const unsigned mask = __ballot_sync(0xffffffffu, valid);
-    if (!valid) return;
-    const unsigned peers = __match_any_sync(mask, c);
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(peers) - 1;
-    const unsigned rank = __popc(peers & ((1u << lane) - 1u));
+    // runs of equal cells among consecutive lanes: one atomic each (lanes past the end: a run with
+    // no cell).  Particles are nearly sorted, so a cell is one run; a cell met again in the warp
+    // only takes a second atomic.
+    const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
+    const unsigned prev = __shfl_up_sync(full, c, 1);
+    const unsigned heads = __ballot_sync(full, lane == 0 || prev != c);
+    const unsigned upto = heads & (full >> (31u - lane));
+    const unsigned head = 31u - (unsigned)__clz((int)upto);
+    const unsigned above = lane < 31u ? heads >> (lane + 1u) : 0u;
+    const unsigned len = above ? (unsigned)__ffs((int)above) : 32u - lane;   // of the run from this lane on
     unsigned base = 0;
-    if (lane == leader) base = atomicAdd(&count[c], (unsigned)__popc(peers));
-    base = __shfl_sync(peers, base, leader);
+    if (lane == head && valid) base = atomicAdd(&count[c], len);
+    base = __shfl_sync(full, base, (int)head);
+    if (!valid) return;
+    const unsigned rank = lane - head;
     sub[i] = base + rank;
     cell_old[i] = c;
     if (bad) atomicAdd(&st->out_of_grid, 1u);
@@ -79,10 +88,14 @@ __global__ void __launch_bounds__(kScanThreads)
 k_scan_reduce(const unsigned *__restrict__ count, unsigned cells, unsigned *__restrict__ partials) {
     const unsigned base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     unsigned s = 0;
+    if (base + kScanItems <= cells && (reinterpret_cast<size_t>(count) & 15u) == 0) {
+        const uint4 a = *reinterpret_cast<const uint4 *>(count + base);
+        const uint4 b = *reinterpret_cast<const uint4 *>(count + base + 4);
+        s = a.x + a.y + a.z + a.w + b.x + b.y + b.z + b.w;
+    } else {
 #pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        unsigned idx = base + k;
-        if (idx < cells) s += count[idx];
+        for (int k = 0; k < kScanItems; k++)
+            if (base + k < cells) s += count[base + k];
     }
     unsigned total;
     block_excl_scan(s, &total);
@@ -102,24 +115,43 @@ k_scan_apply(unsigned *__restrict__ count, unsigned cells, const unsigned *__res
     const unsigned base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     unsigned v[kScanItems];
     unsigned s = 0;
+    // 16-byte accesses: all but the last threads, and arrays that are aligned (a caller's may not be)
+    const bool whole = base + kScanItems <= cells &&
+                       ((reinterpret_cast<size_t>(count) | reinterpret_cast<size_t>(start)) & 15u) == 0;
+    if (whole) {
+        const uint4 a = *reinterpret_cast<const uint4 *>(count + base);
+        const uint4 b = *reinterpret_cast<const uint4 *>(count + base + 4);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
 #pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        unsigned idx = base + k;
-        v[k] = idx < cells ? count[idx] : 0u;
-        s += v[k];
+        for (int k = 0; k < kScanItems; k++) v[k] = base + k < cells ? count[base + k] : 0u;
     }
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) s += v[k];
     unsigned total;
     unsigned run = block_excl_scan(s, &total) + carry;
+    unsigned o[kScanItems];
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        unsigned idx = base + k;
-        if (idx < cells) {
-            start[idx] = run;
-            count[idx] = 0u;   // leave the histogram zeroed for the next update
-            if (idx == cells - 1) start[cells] = run + v[k];
-        }
+        o[k] = run;
         run += v[k];
     }
+    // the counts are left zeroed for the next update
+    if (whole) {
+        *reinterpret_cast<uint4 *>(start + base) = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4 *>(start + base + 4) = make_uint4(o[4], o[5], o[6], o[7]);
+        *reinterpret_cast<uint4 *>(count + base) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4 *>(count + base + 4) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanItems; k++)
+            if (base + k < cells) {
+                start[base + k] = o[k];
+                count[base + k] = 0u;
+            }
+    }
+    if (base < cells && base + kScanItems >= cells) start[cells] = run;
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -132,15 +164,15 @@ k_place(int n, const unsigned *__restrict__ cell_old, const unsigned *__restrict
 }
 
 __global__ void __launch_bounds__(kThreads)
-k_rank_gather(int n, const uint2 *__restrict__ tmp, const unsigned *__restrict__ cell_old,
+k_rank_gather(Params P, const uint2 *__restrict__ tmp, const unsigned *__restrict__ cell_old,
               const unsigned *__restrict__ start, const float4 *__restrict__ pos_in,
               const float4 *__restrict__ vel_in, float4 *__restrict__ pos_out,
               float4 *__restrict__ vel_out, int *__restrict__ pid_out, int *__restrict__ slot,
               unsigned *__restrict__ cell, const float *__restrict__ press_in,
               float *__restrict__ pprev, StepState *st, const float *__restrict__ carry_in,
-              float *__restrict__ carry_out) {
+              float *__restrict__ carry_out, __half *__restrict__ rec) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
+    if (t >= P.n) return;
     const uint2 e = tmp[t];
     const unsigned c = cell_old[e.y];
     const unsigned a = start[c], b = start[c + 1];
@@ -152,13 +184,15 @@ k_rank_gather(int n, const uint2 *__restrict__ tmp, const unsigned *__restrict__
     } else if ((unsigned)t == a) {
         atomicAdd(&st->crowded, 1u);
     }
-    pos_out[dst] = pos_in[e.y];
+    const float4 p = pos_in[e.y];
+    pos_out[dst] = p;
     vel_out[dst] = vel_in[e.y];
     pid_out[dst] = (int)e.x;
     slot[e.x] = (int)dst;
     cell[dst] = c;
     pprev[dst] = press_in[e.y];   // carried for a warm-started corrector
     if (carry_out) carry_out[dst] = carry_in[e.y];
+    filter_record(P, p, c, dst, rec);
 }
 
 size_t scan_partials_needed(unsigned cells) { return (size_t)blocks_for(cells, kScanTile) + 1; }
@@ -190,8 +224,9 @@ void launch_grid_update(const Params &P, const DevBufs &B, int src, int pid_src,
     BBG_PEND(B, s);
     BBG_PBEGIN(B, KID_RANK_GATHER, s, -1);
     k_rank_gather<<<blocks_for(n, kThreads), kThreads, 0, s>>>(
-        n, B.tmp, B.cell_old, B.start, B.pos[src], B.vel[src], B.pos[1 - src], B.vel[1 - src],
-        B.pid[1 - pid_src], B.slot, B.cell, B.press, B.pprev, B.st, carry_in, carry_out);
+        P, B.tmp, B.cell_old, B.start, B.pos[src], B.vel[src], B.pos[1 - src], B.vel[1 - src],
+        B.pid[1 - pid_src], B.slot, B.cell, B.press, B.pprev, B.st, carry_in, carry_out,
+        reinterpret_cast<__half *>(B.frec));
     BBG_PEND(B, s);
 }
 

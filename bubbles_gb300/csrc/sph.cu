@@ -20,8 +20,6 @@
 // iterations after convergence return immediately.
 #include <climits>
 
-#include <cuda_fp16.h>
-
 #include "bbg_kernels.h"
 #include "tile.cuh"
 
@@ -211,45 +209,11 @@ __device__ __forceinline__ void density_members(const Params &P, const float4 *_
     }
 }
 
-// Where the density pass's filter sees a particle of cell (cx, cy, cz): its offset from the
-// cell's lower corner in units of the longest cell side, or NaN when it does not lie in the cell
-// (clamped into the grid, moved since the grid update), which the filter never drops.
-__device__ __forceinline__ v3 filter_offset(const Params &P, float4 p, int cx, int cy, int cz) {
-    const GridDev &g = P.g;
-    const float x = (p.x - (g.minp[0] + (float)cx * g.len[0])) * P.filt_unit;
-    const float y = (p.y - (g.minp[1] + (float)cy * g.len[1])) * P.filt_unit;
-    const float z = (p.z - (g.minp[2] + (float)cz * g.len[2])) * P.filt_unit;
-    const float lo = -P.filt_edge, hi = P.filt_edge;
-    const bool in = x >= lo && x <= P.filt_side[0] + hi && y >= lo && y <= P.filt_side[1] + hi && z >= lo &&
-                    z <= P.filt_side[2] + hi;
-    const float nan = __int_as_float(0x7fffffff);
-    return in ? V(x, y, z) : V(nan, nan, nan);
-}
-
-__device__ __forceinline__ void cell_coords(const GridDev &g, unsigned c, int &cx, int &cy, int &cz) {
-    const unsigned plane = (unsigned)g.nx * (unsigned)g.ny;
-    cz = (int)(c / plane);
-    const unsigned rem = c - (unsigned)cz * plane;
-    cy = (int)(rem / (unsigned)g.nx);
-    cx = (int)(rem - (unsigned)cy * (unsigned)g.nx);
-}
-
-// Positions in half precision for the density pass's filter: slots 8k .. 8k + 7 share a record of
-// four rows of eight halves, x, y, z and x'.  y and z are offsets from the centre of the
-// particle's own cell; x counts cells modulo 4 from the middle of a window of four, x' with the
-// window two cells on, so that the three cells around any cell lie in one of the two windows.
+// The filter's records of positions that the last grid update did not write them for.
 __global__ void __launch_bounds__(kThreads)
 k_filter_records(Params P, const float4 *__restrict__ pos, const unsigned *__restrict__ cell, __half *__restrict__ rec) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n) return;
-    int cx, cy, cz;
-    cell_coords(P.g, cell[i] & ~kWide, cx, cy, cz);
-    const v3 f = filter_offset(P, pos[i], cx, cy, cz);
-    __half *r = rec + 32 * (size_t)(i >> 3) + (i & 7);
-    r[0] = __float2half_rn((float)((cx & 3) - 2) * P.filt_side[0] + f.x);
-    r[8] = __float2half_rn(f.y - 0.5f * P.filt_side[1]);
-    r[16] = __float2half_rn(f.z - 0.5f * P.filt_side[2]);
-    r[24] = __float2half_rn((float)(((cx + 2) & 3) - 2) * P.filt_side[0] + f.x);
+    if (i < P.n) filter_record(P, pos[i], cell[i] & ~kWide, (unsigned)i, rec);
 }
 
 __device__ __forceinline__ unsigned half2_bits(__half2 v) { return *reinterpret_cast<unsigned *>(&v); }
@@ -1080,11 +1044,12 @@ void launch_export_members(const Params &P, const DevBufs &B, int buf, int pid_b
                                                                     B.pid[pid_buf], a, b, maxm, counts, out);
 }
 
-void launch_density(const Params &P, const DevBufs &B, int buf, int compute_pressure, cudaStream_t s) {
+void launch_density(const Params &P, const DevBufs &B, int buf, int compute_pressure, cudaStream_t s, bool recorded) {
     BBG_PBEGIN(B, KID_DENSITY, s, -1);
     const int t = B.tune.block;
-    k_filter_records<<<blocks_for(P.n, kThreads), kThreads, 0, s>>>(P, B.pos[buf], B.cell,
-                                                                    reinterpret_cast<__half *>(B.frec));
+    if (!recorded)
+        k_filter_records<<<blocks_for(P.n, kThreads), kThreads, 0, s>>>(P, B.pos[buf], B.cell,
+                                                                        reinterpret_cast<__half *>(B.frec));
     k_density_mask<<<blocks_for(P.n, t), t, sizeof(uint2) * kMasks * (size_t)t, s>>>(
         P, B.pos[buf], B.vel[buf], B.cell, B.start, B.frec, B.rho, B.inv_rho, B.press, B.nbr, B.list,
         compute_pressure, B.st);

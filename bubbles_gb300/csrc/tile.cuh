@@ -13,6 +13,8 @@
 // Entries are absolute slot indices (32 bit).
 #pragma once
 
+#include <cuda_fp16.h>
+
 #include "bbg_internal.cuh"
 
 namespace bbg {
@@ -36,6 +38,44 @@ __device__ __forceinline__ int tile_of_block(const Params &P, int b, int tiles) 
     if (G <= 0) return b;
     const int per = (tiles + G - 1) / G;
     return (b % G) * per + b / G;
+}
+
+// Where the density pass's filter sees a particle of cell (cx, cy, cz): its offset from the
+// cell's lower corner in units of the longest cell side, or NaN when it does not lie in the cell
+// (clamped into the grid, moved since the grid update), which the filter never drops.
+__device__ __forceinline__ v3 filter_offset(const Params &P, float4 p, int cx, int cy, int cz) {
+    const GridDev &g = P.g;
+    const float x = (p.x - (g.minp[0] + (float)cx * g.len[0])) * P.filt_unit;
+    const float y = (p.y - (g.minp[1] + (float)cy * g.len[1])) * P.filt_unit;
+    const float z = (p.z - (g.minp[2] + (float)cz * g.len[2])) * P.filt_unit;
+    const float lo = -P.filt_edge, hi = P.filt_edge;
+    const bool in = x >= lo && x <= P.filt_side[0] + hi && y >= lo && y <= P.filt_side[1] + hi && z >= lo &&
+                    z <= P.filt_side[2] + hi;
+    const float nan = __int_as_float(0x7fffffff);
+    return in ? V(x, y, z) : V(nan, nan, nan);
+}
+
+__device__ __forceinline__ void cell_coords(const GridDev &g, unsigned c, int &cx, int &cy, int &cz) {
+    const unsigned plane = (unsigned)g.nx * (unsigned)g.ny;
+    cz = (int)(c / plane);
+    const unsigned rem = c - (unsigned)cz * plane;
+    cy = (int)(rem / (unsigned)g.nx);
+    cx = (int)(rem - (unsigned)cy * (unsigned)g.nx);
+}
+
+// Slot i of the density pass's filter: positions in half precision, slots 8k .. 8k + 7 in a record of
+// four rows of eight halves, x, y, z and x'.  y and z are offsets from the centre of the
+// particle's own cell; x counts cells modulo 4 from the middle of a window of four, x' with the
+// window two cells on, so that the three cells around any cell lie in one of the two windows.
+__device__ __forceinline__ void filter_record(const Params &P, float4 p, unsigned c, unsigned i, __half *rec) {
+    int cx, cy, cz;
+    cell_coords(P.g, c, cx, cy, cz);
+    const v3 f = filter_offset(P, p, cx, cy, cz);
+    __half *r = rec + 32 * (size_t)(i >> 3) + (i & 7u);
+    r[0] = __float2half_rn((float)((cx & 3) - 2) * P.filt_side[0] + f.x);
+    r[8] = __float2half_rn(f.y - 0.5f * P.filt_side[1]);
+    r[16] = __float2half_rn(f.z - 0.5f * P.filt_side[2]);
+    r[24] = __float2half_rn((float)(((cx + 2) & 3) - 2) * P.filt_side[0] + f.x);
 }
 
 // The 9 row ranges of the 27 neighbour cells of cell c in z, y, x order: f(r, b, e) for
