@@ -1334,10 +1334,12 @@ bbg_status bbg_advance(bbg_solver s, double dt, bbg_step_stats *stats) {
     if (!(dt > 0)) return fail(BBG_ERR_INVALID_ARGUMENT, "dt must be > 0");
     memset(&s->acc, 0, sizeof(s->acc));
     float remaining = (float)dt;
+    // the largest force of the state at hand; after a substep it comes with its step state, which
+    // the integrating pass reduced, so the CFL loop waits for the device once a substep
+    float mf = 0;
+    bbg_status r = BBG_OK;
+    if (remaining > 0.0001f && (r = max_force(s, &mf))) return r;
     while (remaining > 0.0001f) {   // Epsilon, src/core/geometry.h:44
-        float mf = 0;
-        bbg_status r = max_force(s, &mf);
-        if (r) return r;
         unsigned nsteps = number_of_time_steps(remaining, (float)s->desc.sound_speed,
                                                (float)s->desc.time_step_limit_scale,
                                                s->kernel_radius, s->mass, mf);
@@ -1346,6 +1348,7 @@ bbg_status bbg_advance(bbg_solver s, double dt, bbg_step_stats *stats) {
         if ((r = substep(s, step))) return r;
         if ((r = read_step_state(s))) return r;
         add_substep_stats(s, step);
+        memcpy(&mf, &s->h_st->max_force_bits, 4);
         remaining -= step;
     }
     if (stats) *stats = s->acc;
