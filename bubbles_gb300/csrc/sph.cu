@@ -62,6 +62,14 @@ constexpr int kPfWlMinBlocks = BBG_PFWL_MIN_BLOCKS * kTile / kMaxTile;
 // density pass: 64 registers (measured at 1M particles: 8 and 10 blocks the same, 12 spills)
 constexpr int kDensityMinBlocks = BBG_DENSITY_MIN_BLOCKS * kTile / kMaxTile;
 
+// Up to this many particles the member passes are bound by the latency of each particle's dependent
+// loads, with few warps an SM to hide it: kernels that request more of them together, at up to
+// 128 registers, so four blocks of 128 an SM, and one wave of 152 SMs is the line.  A
+// substep of 19,720 particles, 8 corrector iterations: 218 -> 193 us; 65,600: 222 -> 208; 5,814, 1
+// iteration: 79 -> 71; past the line they lose (122,500: 271 -> 341).
+constexpr int kFew = 152 * 4 * kTile;
+constexpr int kFewBatch = 16, kFewBatchPosVel = 8;   // members together (one or two records each)
+
 // a neighbour's position and velocity records
 struct PosVel {
     float4 p, v;
@@ -169,16 +177,17 @@ __device__ __forceinline__ void density_walk(const Params &P, const float4 *__re
 }
 
 // The member phase over `kept` non-empty masks of candidates, entry k at keep[k * stride]: (mask,
-// slot of bit 31, the next slots below it).  Four records requested together.
+// slot of bit 31, the next slots below it).  NB records requested together.
+template <int NB>
 __device__ __forceinline__ void density_members(const Params &P, const float4 *__restrict__ pos, float4 pi, unsigned i,
                                                 DensitySum &D, const uint2 *keep, int stride, int kept) {
     const uint2 *const end = keep + kept * stride;
     unsigned m = 0, base = 0;
     while (m != 0 || keep != end) {
-        unsigned j[4];
-        bool mem[4];
+        unsigned j[NB];
+        bool mem[NB];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
+        for (int u = 0; u < NB; u++) {
             if (m == 0 && keep != end) {
                 const uint2 v = *keep;
                 m = v.x;
@@ -190,22 +199,22 @@ __device__ __forceinline__ void density_members(const Params &P, const float4 *_
             j[u] = mem[u] ? base + c : i;
             m &= ~(0x80000000u >> c);
         }
-        float4 p[4];
+        float4 p[NB];
 #pragma unroll
-        for (int u = 0; u < 4; u++) p[u] = __ldg(&pos[j[u]]);
-        float r2[4];
+        for (int u = 0; u < NB; u++) p[u] = __ldg(&pos[j[u]]);
+        float r2[NB];
         bool all = true;   // members without the exact test
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
+        for (int u = 0; u < NB; u++) {
             r2[u] = DensitySum::dist(pi, p[u]);
             all = all && r2[u] < P.nb_lo;
         }
         if (!all) {
 #pragma unroll
-            for (int u = 0; u < 4; u++) mem[u] = mem[u] && std_member(P, pi, p[u], r2[u]);
+            for (int u = 0; u < NB; u++) mem[u] = mem[u] && std_member(P, pi, p[u], r2[u]);
         }
 #pragma unroll
-        for (int u = 0; u < 4; u++) D.take(P, mem[u], r2[u], j[u], i);
+        for (int u = 0; u < NB; u++) D.take(P, mem[u], r2[u], j[u], i);
     }
 }
 
@@ -239,7 +248,11 @@ constexpr int kMasks = 10;
 // a clock return 12 bytes a candidate to every lane (181 us), half of that as halves.  A warp per
 // cell that holds candidates in registers and ballots each particle's tests was slower (225 us): the
 // setup per cell, 5.5 cells a warp, costs more than the loads it saves.
-__global__ void __launch_bounds__(kMaxTile, kDensityMinBlocks)
+//
+// FEW (fewer particles than fill the SMs): a row's records are all requested before any is used, and
+// more members together, since no other warp hides their latency.
+template <bool FEW>
+__global__ void __launch_bounds__(kMaxTile, FEW ? 1 : kDensityMinBlocks)
 k_density_mask(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, unsigned *__restrict__ cell,
                const unsigned *__restrict__ start, const uint4 *__restrict__ rec, float *__restrict__ rho,
                float *__restrict__ inv_rho, float *__restrict__ press, int *__restrict__ nbr,
@@ -305,8 +318,7 @@ k_density_mask(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, uns
                 const int groups = (int)((span + 7u) >> 3);
                 const uint4 *q = rec0 + (size_t)(cb >> 3) * 4u;
                 unsigned m = 0;
-                for (int k = 0; k < groups; k++, q += 4) {
-                    const uint4 a = __ldg(q), v = __ldg(q + 1), w = __ldg(q + 2);
+                auto group = [&](const uint4 &a, const uint4 &v, const uint4 &w) {
                     auto test = [&](unsigned ua, unsigned ub, unsigned uc) {
                         const __half2 da = __hsub2(as_half2(ua), A), db = __hsub2(as_half2(ub), B);
                         const __half2 dc = __hsub2(as_half2(uc), C);
@@ -318,6 +330,21 @@ k_density_mask(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, uns
                     unsigned s = __dp4a(__byte_perm(w0, w1, 0x7531) & 0x80808080u, 0x10204080u, 0u);
                     s = __dp4a(__byte_perm(w2, w3, 0x7531) & 0x80808080u, 0x01020408u, s);
                     m = (m << 8) + (s >> 7);
+                };
+                if (FEW) {
+                    uint4 a[4], v[4], w[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const uint4 *g4 = q + 4 * min(k, groups - 1);
+                        a[k] = __ldg(g4);
+                        v[k] = __ldg(g4 + 1);
+                        w[k] = __ldg(g4 + 2);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if (k < groups) group(a[k], v[k], w[k]);
+                } else {
+                    for (int k = 0; k < groups; k++, q += 4) group(__ldg(q), __ldg(q + 1), __ldg(q + 2));
                 }
                 m = ~m << (32 - 8 * groups);
                 // the slots of [b, e) only
@@ -332,7 +359,7 @@ k_density_mask(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, uns
     }
     DensitySum D(list + i);
     if (kept > kMasks || total > kMaxCandidates) density_walk(P, pos, start, c, pi, (unsigned)i, st, D);
-    else density_members(P, pos, pi, (unsigned)i, D, keep, stride, kept);
+    else density_members<FEW ? 8 : 4>(P, pos, pi, (unsigned)i, D, keep, stride, kept);
     density_store(P, pos, vel, cell, rho, inv_rho, press, nbr, compute_pressure, st, i, pi, cw, D.sum,
                   D.listed + D.self, D.listed);
 }
@@ -345,8 +372,8 @@ k_density_mask(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, uns
 //   (PredictPressureForceFor, pcisph_equations3.cpp:114-155) and x* comes from F + Fp.
 // With DIV it also accumulates sum_j (1/rho_j) (1 - d/h)^2 / d (v_j - v_i).(x_j - x_i),
 // the velocity divergence up to m * 45 / (pi h^4), a feature of the learned warm start.
-template <bool DIV, bool WARM, int NB>
-__global__ void __launch_bounds__(kMaxTile, kNbrMinBlocks)
+template <bool DIV, bool WARM, int NB, int MINB = kNbrMinBlocks>
+__global__ void __launch_bounds__(kMaxTile, MINB)
 k_non_pressure(Params P, const float4 *__restrict__ pos, const float4 *__restrict__ vel,
                const unsigned *__restrict__ cell,
                const unsigned *__restrict__ start, const ListEntry *__restrict__ list, const int *__restrict__ nbr,
@@ -623,8 +650,8 @@ __device__ __forceinline__ int block_tile(const Params &P, int wl, int slots) {
 
 // One block per tile (all tiles, or the work list's) of PPT x blockDim slots; thread t
 // takes slots t, t + blockDim, ... (PPT particles per thread).
-template <int NB, int PPT>
-__global__ void __launch_bounds__(kMaxTile, kPdMinBlocks)
+template <int NB, int PPT, int MINB = kPdMinBlocks>
+__global__ void __launch_bounds__(kMaxTile, MINB)
 k_pred_density(Params P, float4 *pos, const float4 *__restrict__ xstar,
                const unsigned *__restrict__ cell, const unsigned *__restrict__ start,
                const ListEntry *__restrict__ list, const int *__restrict__ nbr, float *__restrict__ press,
@@ -742,8 +769,8 @@ __device__ __forceinline__ bool corrector_ends(const Params &P, const StepState 
                          fdv(__uint_as_float(st->err_bits[k]), P.target_density) < P.max_err_ratio);
 }
 
-template <int NB, int PPT>
-__global__ void __launch_bounds__(kMaxTile, kPfMinBlocks)
+template <int NB, int PPT, int MINB = kPfMinBlocks>
+__global__ void __launch_bounds__(kMaxTile, MINB)
 k_pressure_force(Params P, const float4 *__restrict__ pos, const float4 *__restrict__ vel,
                  const unsigned *__restrict__ cell, const unsigned *__restrict__ start,
                  const ListEntry *__restrict__ list, const int *__restrict__ nbr, float4 *__restrict__ force,
@@ -884,6 +911,7 @@ k_worklist(Params P, const StepState *st, int k, int tile) {
 // reference integrates each particle inside the force loop (:277), racing with its
 // neighbours' reads; here all forces read the step-start state and the integrated
 // state goes to the other buffer.
+template <int NB>
 __global__ void __launch_bounds__(kMaxTile)
 k_sph_forces(Params P, const float4 *__restrict__ pos, const float4 *__restrict__ vel,
              const unsigned *__restrict__ cell, const unsigned *__restrict__ start,
@@ -902,7 +930,7 @@ k_sph_forces(Params P, const float4 *__restrict__ pos, const float4 *__restrict_
         float tx = 0.f, ty = 0.f, tz = 0.f;
         const float kg = P.m2 * P.spiky_dw_c;
         const float kv = P.visc_m2 * P.spiky_d2w_c;
-        tile_members<(kGatherBatch < 4 ? kGatherBatch : 4)>(
+        tile_members<NB>(
             P, start, list, nbr, pos, cell[i], i,
             [&](unsigned j) { return PosVel{__ldg(&pos[j]), __ldg(&vel[j])}; },
             [&](const PosVel &nb) {
@@ -1050,7 +1078,8 @@ void launch_density(const Params &P, const DevBufs &B, int buf, int compute_pres
     if (!recorded)
         k_filter_records<<<blocks_for(P.n, kThreads), kThreads, 0, s>>>(P, B.pos[buf], B.cell,
                                                                         reinterpret_cast<__half *>(B.frec));
-    k_density_mask<<<blocks_for(P.n, t), t, sizeof(uint2) * kMasks * (size_t)t, s>>>(
+    const auto density = P.n <= kFew ? k_density_mask<true> : k_density_mask<false>;
+    density<<<blocks_for(P.n, t), t, sizeof(uint2) * kMasks * (size_t)t, s>>>(
         P, B.pos[buf], B.vel[buf], B.cell, B.start, B.frec, B.rho, B.inv_rho, B.press, B.nbr, B.list,
         compute_pressure, B.st);
     if (P.nscenes > 0 && P.n > 0) {
@@ -1083,11 +1112,12 @@ static void non_pressure_nb(const Params &P0, const DevBufs &B, int buf, int pre
     const int t = B.tune.block;
     Params P;
     const int grid = tiled_grid(P0, B, t, &P);
-#define NP_LAUNCH(NB)                                                                        \
-    k_non_pressure<DIV, WARM, NB><<<grid, t, 0, s>>>(                                        \
+#define NP_LAUNCH(...)                                                                       \
+    k_non_pressure<DIV, WARM, __VA_ARGS__><<<grid, t, 0, s>>>(                                        \
         P, B.pos[buf], B.vel[buf], B.cell, B.start, B.list, B.nbr, B.force, B.xstar, B.pforce, \
         B.press, divsum, predict, dt, dt_over_m)
-    switch (B.tune.batch_np) {
+    if (P.n <= kFew) NP_LAUNCH(kFewBatchPosVel, 1);
+    else switch (B.tune.batch_np) {
         case 2: NP_LAUNCH(2); break;
         case 8: NP_LAUNCH(8); break;
         default: NP_LAUNCH(4); break;
@@ -1138,17 +1168,17 @@ void update_worklist_grid(DevBufs &B) {
     B.tune.wl_grid_pf = B.tune.batch_pf == 2 ? pf_grid<2>(t) : B.tune.batch_pf == 8 ? pf_grid<8>(t) : pf_grid<4>(t);
 }
 
-// Particles per thread of the per-tile corrector passes.
-static int corrector_ppt(const DevBufs &B) { return B.tune.ppt == 2 ? 2 : 1; }
+// Particles per thread of the per-tile corrector passes (few particles: one).
+static int corrector_ppt(const Params &P, const DevBufs &B) { return B.tune.ppt == 2 && P.n > kFew ? 2 : 1; }
 
 // Slots per tile of the corrector passes: the block, times the particles per thread for
 // the per-tile kernels.
-static int corrector_tile(const DevBufs &B) {
-    return B.tune.block * (B.tune.worklist == 2 ? 1 : corrector_ppt(B));
+static int corrector_tile(const Params &P, const DevBufs &B) {
+    return B.tune.block * (B.tune.worklist == 2 ? 1 : corrector_ppt(P, B));
 }
 
 void launch_worklist(const Params &P, const DevBufs &B, int k, cudaStream_t s) {
-    k_worklist<<<1, 1024, 0, s>>>(P, B.st, k, corrector_tile(B));
+    k_worklist<<<1, 1024, 0, s>>>(P, B.st, k, corrector_tile(P, B));
 }
 
 void launch_pred_density(const Params &P, const DevBufs &B, int buf, int k, float delta,
@@ -1170,14 +1200,15 @@ void launch_pred_density(const Params &P, const DevBufs &B, int buf, int k, floa
         }
 #undef PD_LAUNCH
     } else {
-        const int ppt = corrector_ppt(B);
+        const int ppt = corrector_ppt(P, B);
         Params Q;
         const int grid = wl ? blocks_for(P.n, t * ppt) : tiled_grid(P, B, t * ppt, &Q);
         if (wl) Q = P;
-#define PD_LAUNCH(NB, PPT)                                                                        \
-    k_pred_density<NB, PPT><<<grid, t, 0, s>>>(Q, B.pos[buf], B.xstar, B.cell, B.start, B.list, B.nbr, \
+#define PD_LAUNCH(...)                                                                            \
+    k_pred_density<__VA_ARGS__><<<grid, t, 0, s>>>(Q, B.pos[buf], B.xstar, B.cell, B.start, B.list, B.nbr, \
                                                B.press, B.rhostar, B.derr, B.st, k, delta, clamp_total, wl)
-        switch (B.tune.batch_pd * 10 + ppt) {
+        if (P.n <= kFew) PD_LAUNCH(kFewBatch, 1, 1);
+        else switch (B.tune.batch_pd * 10 + ppt) {
             case 21: PD_LAUNCH(2, 1); break;
             case 81: PD_LAUNCH(8, 1); break;
             case 22: PD_LAUNCH(2, 2); break;
@@ -1219,15 +1250,16 @@ void launch_pressure_force(const Params &P, const DevBufs &B, int buf, int k, in
         }
 #undef PF_LAUNCH
     } else {
-        const int ppt = corrector_ppt(B);
+        const int ppt = corrector_ppt(P, B);
         Params Q;
         const int grid = wl ? blocks_for(P.n, t * ppt) : tiled_grid(P, B, t * ppt, &Q);
         if (wl) Q = P;
-#define PF_LAUNCH(NB, PPT)                                                                             \
-    k_pressure_force<NB, PPT><<<grid, t, 0, s>>>(                                                       \
+#define PF_LAUNCH(...)                                                                                 \
+    k_pressure_force<__VA_ARGS__><<<grid, t, 0, s>>>(                                                       \
         Q, B.pos[buf], B.vel[buf], B.cell, B.start, B.list, B.nbr, B.force, B.pforce, B.xstar,           \
         B.pos[1 - buf], B.vel[1 - buf], B.st, k, max_it, dt, dt_over_m, mode, wl, loop)
-        switch (B.tune.batch_pf * 10 + ppt) {
+        if (P.n <= kFew) PF_LAUNCH(kFewBatch, 1, 1);
+        else switch (B.tune.batch_pf * 10 + ppt) {
             case 21: PF_LAUNCH(2, 1); break;
             case 81: PF_LAUNCH(8, 1); break;
             case 22: PF_LAUNCH(2, 2); break;
@@ -1242,7 +1274,8 @@ void launch_pressure_force(const Params &P, const DevBufs &B, int buf, int k, in
 
 void launch_sph_forces(const Params &P, const DevBufs &B, int buf, float dt, cudaStream_t s) {
     BBG_PBEGIN(B, KID_SPH_FORCES, s, -1);
-    k_sph_forces<<<blocks_for(P.n, B.tune.block), B.tune.block, 0, s>>>(
+    const auto forces = P.n <= kFew ? k_sph_forces<kFewBatchPosVel> : k_sph_forces<(kGatherBatch < 4 ? kGatherBatch : 4)>;
+    forces<<<blocks_for(P.n, B.tune.block), B.tune.block, 0, s>>>(
         P, B.pos[buf], B.vel[buf], B.cell, B.start, B.list, B.nbr, B.force, B.pos[1 - buf],
         B.vel[1 - buf], B.st, dt);
     BBG_PEND(B, s);
