@@ -228,26 +228,36 @@ __global__ void k_mlp_collect(int n, int batch, const unsigned *__restrict__ ste
 // its tiles' weight gradients into its own row of gpart and their (weighted) squared
 // errors into lpart[block], always in the same order, so training is deterministic (no
 // atomics; the Adam kernel adds the rows in block order).
-__global__ void __launch_bounds__(128)
+//
+// The three products with the 64 x 64 layer are FP32 matrix products in shared memory with the
+// operands of 32 accumulators (16 for the weight gradient) a thread in registers: 3 to 12
+// 16-byte loads per 32 to 128 fma, activations as rows of 128 samples padded to 132 so that rows
+// side by side fall in other banks.  A thread per sample that read a weight or an activation for
+// every fma was bound by shared memory (16-way conflicts in the weight gradient): 57 us for
+// 16,384 pairs, 29 us now (its gradients read by Adam in 11 us instead of 16).  Every sum runs in the same order as there.
+constexpr int kTrainThreads = 256, kTrainStride = 132;
+
+__global__ void __launch_bounds__(kTrainThreads)
 k_mlp_train(int batch, const float4 *__restrict__ bx, const float *__restrict__ bt,
             const float *__restrict__ theta, float *__restrict__ gpart, double *__restrict__ lpart,
             float expectile) {
-    extern __shared__ float smem[];
-    float *sW2 = smem;                    // [64][64]
-    float *sW1 = sW2 + kHid * kHid;       // [4][64]
+    extern __shared__ float4 train_smem[];
+    constexpr int S = kTrainStride;
+    float *sW2 = reinterpret_cast<float *>(train_smem);   // [64][64]
+    float *sH1 = sW2 + kHid * kHid;       // [64][S]
+    float *sD1 = sH1 + kHid * S;          // [64][S]  GELU'(z1), then dz1
+    float *sH2 = sD1 + kHid * S;          // [64][S]
+    float *sD2 = sH2 + kHid * S;          // [64][S]  GELU'(z2), then dz2
+    float *sX = sD2 + kHid * S;           // [4][S]
+    float *sW1 = sX + kIn * S;            // [4][64]
     float *sB1 = sW1 + kIn * kHid;        // [64]
     float *sB2 = sB1 + kHid;              // [64]
     float *sW3 = sB2 + kHid;              // [64]
-    float *sX = sW3 + kHid;               // [4][128]
-    float *sH1 = sX + kIn * 128;          // [64][128]
-    float *sD1 = sH1 + kHid * 128;        // [64][128]
-    float *sH2 = sD1 + kHid * 128;        // [64][128]
-    float *sD2 = sH2 + kHid * 128;        // [64][128]
-    float *sDY = sD2 + kHid * 128;        // [128]
+    float *sDY = sW3 + kHid;              // [128]
     __shared__ double sLoss[4];
-    const int t = threadIdx.x;
-    for (int k = t; k < kHid * kHid; k += 128) sW2[k] = theta[kOffW2 + k];
-    for (int k = t; k < kIn * kHid; k += 128) sW1[k] = theta[kOffW1 + k];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    for (int k = t; k < kHid * kHid; k += kTrainThreads) sW2[k] = theta[kOffW2 + k];
+    for (int k = t; k < kIn * kHid; k += kTrainThreads) sW1[k] = theta[kOffW1 + k];
     if (t < kHid) {
         sB1[t] = theta[kOffB1 + t];
         sB2[t] = theta[kOffB2 + t];
@@ -256,20 +266,22 @@ k_mlp_train(int batch, const float4 *__restrict__ bx, const float *__restrict__ 
     __syncthreads();
     const float b3 = theta[kOffB3];
     float *grad = gpart + (size_t)blockIdx.x * kParams;
+    const auto row4 = [](float *p) -> float4 & { return *reinterpret_cast<float4 *>(p); };
     for (int tile = blockIdx.x; tile * 128 < batch; tile += gridDim.x) {
         const bool first = tile == (int)blockIdx.x;
         // a block's own gradient row: the first tile stores, later tiles add (same thread)
         auto put = [&](int idx, float v) { grad[idx] = first ? v : grad[idx] + v; };
-        const int s = tile * 128 + t;
+        // layer 1: thread -> sample t mod 128, half of the units
+        const int q = t & 127, s = tile * 128 + q;
         const bool valid = s < batch;
         const float4 x = valid ? bx[s] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float target = valid ? bt[s] : 0.f;
-        sX[0 * 128 + t] = x.x;
-        sX[1 * 128 + t] = x.y;
-        sX[2 * 128 + t] = x.z;
-        sX[3 * 128 + t] = x.w;
-        // forward
-        for (int a = 0; a < kHid; a++) {
+        if (t < 128) {
+            sX[0 * S + q] = x.x;
+            sX[1 * S + q] = x.y;
+            sX[2 * S + q] = x.z;
+            sX[3 * S + q] = x.w;
+        }
+        for (int a = (t >> 7) * (kHid / 2), e = a + kHid / 2; a < e; a++) {
             float z = sB1[a];
             z = fmaf(x.x, sW1[0 * kHid + a], z);
             z = fmaf(x.y, sW1[1 * kHid + a], z);
@@ -277,101 +289,161 @@ k_mlp_train(int batch, const float4 *__restrict__ bx, const float *__restrict__ 
             z = fmaf(x.w, sW1[3 * kHid + a], z);
             float h, d;
             gelu_grad(z, &h, &d);
-            sH1[a * 128 + t] = h;
-            sD1[a * 128 + t] = d;
+            sH1[a * S + q] = h;
+            sD1[a * S + q] = d;
         }
-        float z2[kHid];
-    #pragma unroll
-        for (int k = 0; k < kHid; k++) z2[k] = sB2[k];
+        __syncthreads();
+        // layer 2: warp -> units 8 w .. 8 w + 7, lane -> samples 4 lane .. 4 lane + 3
+        float acc[8][4];
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+#pragma unroll
+            for (int u = 0; u < 4; u++) acc[k][u] = sB2[8 * w + k];
+#pragma unroll 4
         for (int a = 0; a < kHid; a++) {
-            const float h = sH1[a * 128 + t];
-    #pragma unroll
-            for (int k = 0; k < kHid; k++) z2[k] = fmaf(h, sW2[a * kHid + k], z2[k]);
+            const float4 h = row4(sH1 + a * S + 4 * lane);
+            const float4 w0 = row4(sW2 + a * kHid + 8 * w), w1 = row4(sW2 + a * kHid + 8 * w + 4);
+            const float wk[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                acc[k][0] = fmaf(h.x, wk[k], acc[k][0]);
+                acc[k][1] = fmaf(h.y, wk[k], acc[k][1]);
+                acc[k][2] = fmaf(h.z, wk[k], acc[k][2]);
+                acc[k][3] = fmaf(h.w, wk[k], acc[k][3]);
+            }
         }
-        float y = b3;
-    #pragma unroll
-        for (int k = 0; k < kHid; k++) {
-            float h, d;
-            gelu_grad(z2[k], &h, &d);
-            sH2[k * 128 + t] = h;
-            y = fmaf(sW3[k], h, y);
-            z2[k] = d;   // keep GELU'(z2)
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            float4 h;
+            gelu_grad(acc[k][0], &h.x, &acc[k][0]);   // keep GELU'(z2)
+            gelu_grad(acc[k][1], &h.y, &acc[k][1]);
+            gelu_grad(acc[k][2], &h.z, &acc[k][2]);
+            gelu_grad(acc[k][3], &h.w, &acc[k][3]);
+            row4(sH2 + (8 * w + k) * S + 4 * lane) = h;
         }
-        const float err = valid ? y - target : 0.f;
-        // asymmetric squared error (expectile tau): over-estimates weigh (1 - tau) / 0.5,
-        // under-estimates tau / 0.5; tau = 0.5 is the mean squared error
-        const float wgt = (err > 0.f ? 1.f - expectile : expectile) * 2.f;
-        const float dy = 2.f * wgt * err / (float)batch;
-        sDY[t] = dy;
-        // backward through layer 3 and GELU 2
-    #pragma unroll
-        for (int k = 0; k < kHid; k++) {
-            z2[k] = dy * sW3[k] * z2[k];   // dz2
-            sD2[k * 128 + t] = z2[k];
+        __syncthreads();
+        // layer 3 and the error: thread -> sample
+        if (t < 128) {
+            float y = b3;
+#pragma unroll 8
+            for (int k = 0; k < kHid; k++) y = fmaf(sW3[k], sH2[k * S + t], y);
+            const float err = valid ? y - bt[s] : 0.f;
+            // asymmetric squared error (expectile tau): over-estimates weigh (1 - tau) / 0.5,
+            // under-estimates tau / 0.5; tau = 0.5 is the mean squared error
+            const float wgt = (err > 0.f ? 1.f - expectile : expectile) * 2.f;
+            sDY[t] = 2.f * wgt * err / (float)batch;
+            double l = (double)wgt * (double)err * (double)err;
+            for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+            if (lane == 0) sLoss[w] = l;
         }
-        // backward through layer 2 and GELU 1
-        for (int a = 0; a < kHid; a++) {
-            float acc = 0.f;
-    #pragma unroll
-            for (int k = 0; k < kHid; k++) acc = fmaf(sW2[a * kHid + k], z2[k], acc);
-            sD1[a * 128 + t] *= acc;   // dz1
-        }
-        // squared error of the block
-        double l = (double)wgt * (double)err * (double)err;
-        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-        if ((t & 31) == 0) sLoss[t >> 5] = l;
         __syncthreads();
         if (t == 0) {
             const double bl = sLoss[0] + sLoss[1] + sLoss[2] + sLoss[3];
             lpart[blockIdx.x] = first ? bl : lpart[blockIdx.x] + bl;
         }
-        // dW2[a][k] = sum_s h1[a][s] dz2[k][s]: thread -> row a = t / 2, 32 columns
+        // backward through layer 3 and GELU 2
         {
-            const int a = t >> 1, k0 = (t & 1) * 32;
-            float acc[32];
-    #pragma unroll
-            for (int kk = 0; kk < 32; kk++) acc[kk] = 0.f;
-            for (int q = 0; q < 128; q++) {
-                const float h = sH1[a * 128 + q];
-    #pragma unroll
-                for (int kk = 0; kk < 32; kk++) acc[kk] = fmaf(h, sD2[(k0 + kk) * 128 + q], acc[kk]);
+            const float4 dy = row4(sDY + 4 * lane);
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const float w3 = sW3[8 * w + k];
+                row4(sD2 + (8 * w + k) * S + 4 * lane) = make_float4(dy.x * w3 * acc[k][0], dy.y * w3 * acc[k][1],
+                                                                     dy.z * w3 * acc[k][2], dy.w * w3 * acc[k][3]);
             }
-    #pragma unroll
-            for (int kk = 0; kk < 32; kk++) put(kOffW2 + a * kHid + k0 + kk, acc[kk]);
         }
-        // dW1[f][a] = sum_s x[f][s] dz1[a][s]: thread -> a = t / 2, f = 2 (t & 1) + {0, 1}
+        __syncthreads();
+        // backward through layer 2 and GELU 1: warp -> units 8 w .. of layer 1
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+#pragma unroll
+            for (int u = 0; u < 4; u++) acc[k][u] = 0.f;
+#pragma unroll 2
+        for (int k0 = 0; k0 < kHid; k0 += 4) {
+            float4 d[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) d[k] = row4(sD2 + (k0 + k) * S + 4 * lane);
+#pragma unroll
+            for (int a = 0; a < 8; a++) {
+                const float4 wk = row4(sW2 + (8 * w + a) * kHid + k0);
+                const float v[4] = {wk.x, wk.y, wk.z, wk.w};
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    acc[a][0] = fmaf(v[k], d[k].x, acc[a][0]);
+                    acc[a][1] = fmaf(v[k], d[k].y, acc[a][1]);
+                    acc[a][2] = fmaf(v[k], d[k].z, acc[a][2]);
+                    acc[a][3] = fmaf(v[k], d[k].w, acc[a][3]);
+                }
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 8; a++) {
+            float4 &d = row4(sD1 + (8 * w + a) * S + 4 * lane);   // dz1
+            d = make_float4(d.x * acc[a][0], d.y * acc[a][1], d.z * acc[a][2], d.w * acc[a][3]);
+        }
+        // dW2[a][k] = sum_s h1[a][s] dz2[k][s]: thread -> rows a = t mod 16 + 16 u, k = t / 16 + 16 u
         {
-            const int a = t >> 1, f0 = (t & 1) * 2;
-            float g0 = 0.f, g1 = 0.f;
+            const int ra = t & 15, rk = t >> 4;
+            float g[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+#pragma unroll
+                for (int v = 0; v < 4; v++) g[u][v] = 0.f;
+            for (int q0 = 0; q0 < 128; q0 += 4) {
+                float4 h[4], d[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    h[u] = row4(sH1 + (ra + 16 * u) * S + q0);
+                    d[u] = row4(sD2 + (rk + 16 * u) * S + q0);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+#pragma unroll
+                    for (int v = 0; v < 4; v++) {
+                        g[u][v] = fmaf(h[u].x, d[v].x, g[u][v]);
+                        g[u][v] = fmaf(h[u].y, d[v].y, g[u][v]);
+                        g[u][v] = fmaf(h[u].z, d[v].z, g[u][v]);
+                        g[u][v] = fmaf(h[u].w, d[v].w, g[u][v]);
+                    }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+#pragma unroll
+                for (int v = 0; v < 4; v++) put(kOffW2 + (ra + 16 * u) * kHid + rk + 16 * v, g[u][v]);
+        }
+        __syncthreads();
+        // dW1[f][a] = sum_s x[f][s] dz1[a][s]: thread -> a = t / 4, f = t mod 4; these sums and the
+        // biases' start at a sample of their own (no bank conflicts)
+        {
+            const int a = t >> 2, f = t & 3, from = 2 * a + (f >> 1);
+            float g0 = 0.f;
             for (int q0 = 0; q0 < 128; q0++) {
-                const int q = (q0 + t) & 127;
-                const float d = sD1[a * 128 + q];
-                g0 = fmaf(sX[f0 * 128 + q], d, g0);
-                g1 = fmaf(sX[(f0 + 1) * 128 + q], d, g1);
+                const int r = (q0 + from) & 127;
+                g0 = fmaf(sX[f * S + r], sD1[a * S + r], g0);
             }
-            put(kOffW1 + f0 * kHid + a, g0);
-            put(kOffW1 + (f0 + 1) * kHid + a, g1);
+            put(kOffW1 + f * kHid + a, g0);
         }
-        // bias and layer-3 gradients: rows summed with a rotated start (no bank conflicts)
+        // bias and layer-3 gradients
         if (t < kHid) {
-            float gb2 = 0.f, gw3 = 0.f;
-            for (int q0 = 0; q0 < 128; q0++) {
-                const int q = (q0 + t) & 127;
-                gb2 += sD2[t * 128 + q];
-                gw3 = fmaf(sH2[t * 128 + q], sDY[q], gw3);
-            }
+            float gb2 = 0.f;
+            for (int q0 = 0; q0 < 128; q0++) gb2 += sD2[t * S + ((q0 + t) & 127)];
             put(kOffB2 + t, gb2);
-            put(kOffW3 + t, gw3);
-        } else {
+        } else if (t < 2 * kHid) {
             const int a = t - kHid;
             float gb1 = 0.f;
-            for (int q0 = 0; q0 < 128; q0++) gb1 += sD1[a * 128 + ((q0 + t) & 127)];
+            for (int q0 = 0; q0 < 128; q0++) gb1 += sD1[a * S + ((q0 + t) & 127)];
             put(kOffB1 + a, gb1);
-        }
-        if (t < 32) {
-            float gb3 = sDY[t] + sDY[t + 32] + sDY[t + 64] + sDY[t + 96];
+        } else if (t < 3 * kHid) {
+            const int a = t - 2 * kHid;
+            float gw3 = 0.f;
+            for (int q0 = 0; q0 < 128; q0++) {
+                const int r = (q0 + a) & 127;
+                gw3 = fmaf(sH2[a * S + r], sDY[r], gw3);
+            }
+            put(kOffW3 + a, gw3);
+        } else if (t < 3 * kHid + 32) {
+            float gb3 = sDY[lane] + sDY[lane + 32] + sDY[lane + 64] + sDY[lane + 96];
             for (int o = 16; o > 0; o >>= 1) gb3 += __shfl_xor_sync(0xffffffffu, gb3, o);
-            if (t == 0) put(kOffB3, gb3);
+            if (lane == 0) put(kOffB3, gb3);
         }
         __syncthreads();   // the tile's shared rows are rewritten by the next tile
     }
@@ -379,19 +451,25 @@ k_mlp_train(int batch, const float4 *__restrict__ bx, const float *__restrict__ 
 
 // Adam on the FP32 master parameters (bias corrections from the device step counter); the
 // gradient is the sum of the training blocks' rows in block order, the batch loss the sum
-// of their partial losses in block order.
+// of their partial losses in block order (by a block of its own).  A warp a block: the 142 warps
+// on 142 SMs, 16 rows of a parameter requested together.
 __global__ void k_mlp_adam(float *__restrict__ theta, const float *__restrict__ gpart, int rows,
                            const double *__restrict__ lpart, double *__restrict__ loss, float *__restrict__ m1,
                            float *__restrict__ m2, const unsigned *__restrict__ step, float lr, float beta1,
                            float beta2, float eps) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p == 0) {
-        double l = 0.0;
-        for (int b = 0; b < rows; b++) l += lpart[b];
-        *loss += l;
+    if (blockIdx.x == gridDim.x - 1) {
+        if (threadIdx.x == 0) {
+            double l = 0.0;
+#pragma unroll 16
+            for (int b = 0; b < rows; b++) l += lpart[b];
+            *loss += l;
+        }
+        return;
     }
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= kParams) return;
     float gr = 0.f;
+#pragma unroll 16
     for (int b = 0; b < rows; b++) gr += gpart[(size_t)b * kParams + p];
     const float a = beta1 * m1[p] + (1.f - beta1) * gr;
     const float b = beta2 * m2[p] + (1.f - beta2) * gr * gr;
@@ -405,11 +483,12 @@ __global__ void k_mlp_adam(float *__restrict__ theta, const float *__restrict__ 
 
 // BF16 B fragments of the tensor-core layers and the FP32 tail from the master
 // parameters; advances the training step counter.
+constexpr int kPackThreads = 128;
 __global__ void k_mlp_pack(const float *__restrict__ theta, uint32_t *__restrict__ w1f,
                            uint32_t *__restrict__ w2f, float *__restrict__ tail, unsigned *step, int advance) {
-    const int tid = threadIdx.x;   // one block of 256 threads
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;   // a fragment each
     // layer 1: [W1 (rows 0-3); b1 (row 4); 0] as 16 x 64, lane's b0 of n-tile nt
-    for (int k = tid; k < 8 * 32; k += blockDim.x) {
+    for (int k = tid; k < 8 * 32; k += all) {
         const int nt = k / 32, lane = k % 32, g = lane >> 2, t = lane & 3;
         const int col = 8 * nt + g;
         auto w1 = [&](int r) -> float {   // c W1, c b1 (the folded GELU)
@@ -420,13 +499,13 @@ __global__ void k_mlp_pack(const float *__restrict__ theta, uint32_t *__restrict
         w1f[k] = pack_bf16(w1(2 * t), w1(2 * t + 1));
     }
     // layer 2: W2 [64 (k)][64 (n)], fragments (k-chunk kc, n-tile nt, half hh)
-    for (int k = tid; k < 64 * 32; k += blockDim.x) {
+    for (int k = tid; k < 64 * 32; k += all) {
         const int q = k / 32, lane = k % 32, g = lane >> 2, t = lane & 3;
         const int kc = q / 16, nt = (q / 2) % 8, hh = q & 1;
         const int row = 16 * kc + 8 * hh + 2 * t, col = 8 * nt + g;
         w2f[k] = pack_bf16(0.5f * theta[kOffW2 + row * kHid + col], 0.5f * theta[kOffW2 + (row + 1) * kHid + col]);
     }
-    for (int k = tid; k < kHid; k += blockDim.x) {
+    for (int k = tid; k < kHid; k += all) {
         tail[kTailB2 + k] = kGeluC * theta[kOffB2 + k];
         tail[kTailW3 + k] = __bfloat162float(__float2bfloat16_rn((0.5f / kGeluC) * theta[kOffW3 + k]));
     }
@@ -471,7 +550,7 @@ void launch_mlp_infer_raw(const MlpBufs &M, const float4 *feat, int n, float *ou
 }
 
 size_t mlp_train_smem() {
-    return sizeof(float) * ((size_t)kHid * kHid + kIn * kHid + 3 * kHid + kIn * 128 + 4 * kHid * 128 + 128);
+    return sizeof(float) * ((size_t)kHid * kHid + (4 * kHid + kIn) * kTrainStride + kIn * kHid + 3 * kHid + 128);
 }
 
 cudaError_t mlp_prepare() {
@@ -482,10 +561,10 @@ cudaError_t mlp_prepare() {
 void launch_mlp_train_step(const MlpBufs &M, const float4 *bx, const float *bt, int batch, float lr,
                            float beta1, float beta2, float eps, float expectile, cudaStream_t s) {
     const int rows = std::min(blocks_for(batch, 128), kGradRows);
-    k_mlp_train<<<rows, 128, mlp_train_smem(), s>>>(batch, bx, bt, M.theta, M.grad, M.lpart, expectile);
-    k_mlp_adam<<<blocks_for(kParams, 256), 256, 0, s>>>(M.theta, M.grad, rows, M.lpart, M.loss, M.m1, M.m2,
+    k_mlp_train<<<rows, kTrainThreads, mlp_train_smem(), s>>>(batch, bx, bt, M.theta, M.grad, M.lpart, expectile);
+    k_mlp_adam<<<blocks_for(kParams, 32) + 1, 32, 0, s>>>(M.theta, M.grad, rows, M.lpart, M.loss, M.m1, M.m2,
                                                          M.step, lr, beta1, beta2, eps);
-    k_mlp_pack<<<1, 256, 0, s>>>(M.theta, M.w1f, M.w2f, M.tail, M.step, 1);
+    k_mlp_pack<<<64 * 32 / kPackThreads, kPackThreads, 0, s>>>(M.theta, M.w1f, M.w2f, M.tail, M.step, 1);
 }
 
 void launch_mlp_collect(const Params &P, const DevBufs &B, const MlpBufs &M, float p_unit, cudaStream_t s) {
@@ -509,7 +588,7 @@ void launch_mlp_get_features(const MlpBufs &M, const int *slot, float *out, int 
 }
 
 void launch_mlp_pack(const MlpBufs &M, cudaStream_t s) {
-    k_mlp_pack<<<1, 256, 0, s>>>(M.theta, M.w1f, M.w2f, M.tail, M.step, 0);
+    k_mlp_pack<<<64 * 32 / kPackThreads, kPackThreads, 0, s>>>(M.theta, M.w1f, M.w2f, M.tail, M.step, 0);
 }
 
 }  // namespace bbg
