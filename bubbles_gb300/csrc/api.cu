@@ -188,7 +188,7 @@ void free_fields(bbg_solver s) {
 
 void free_frame(bbg_solver s) {
     FrameBufs &F = s->frame;
-    void *ptrs[] = {F.lines, F.lens, F.scan_in, F.offset, F.partials, F.out};
+    void *ptrs[] = {F.lines, F.lens, F.offset, F.partials, F.out};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     F = FrameBufs();

@@ -20,11 +20,11 @@ bbg_status frame_build(bbg_solver s, int flags, std::string *head, size_t *body)
         free_frame(s);
         const size_t n = (size_t)s->capacity;
         bbg_status r = BBG_OK;
-        if (!r) r = dalloc(&F.lines, n * kFrameLineCap);
-        if (!r) r = dalloc(&F.lens, n);
-        if (!r) r = dalloc(&F.scan_in, n);
-        if (!r) r = dalloc(&F.offset, n + 1);
-        if (!r) r = dalloc(&F.partials, scan_partials_needed((unsigned)n));
+        const size_t blocks = (size_t)frame_blocks(s->capacity);
+        if (!r) r = dalloc(&F.lines, blocks * kFrameBlock * kFrameLineCap + 16);   // the last word's neighbour
+        if (!r) r = dalloc(&F.lens, blocks);
+        if (!r) r = dalloc(&F.offset, blocks + 1);
+        if (!r) r = dalloc(&F.partials, scan_partials_needed((unsigned)blocks));
         if (!r) r = dalloc(&F.out, n * kFrameLineCap);
         if (r) {
             free_frame(s);
@@ -35,7 +35,7 @@ bbg_status frame_build(bbg_solver s, int flags, std::string *head, size_t *body)
     launch_frame_lines(s->n, flags, s->B.pos[s->state], s->B.vel[s->state], s->B.rho, s->B.slot, s->mass, F,
                        s->stream);
     CK_LAUNCH();
-    CK(cudaMemcpyAsync(s->h_u, &F.offset[s->n], sizeof(unsigned), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(s->h_u, &F.offset[frame_blocks(s->n)], sizeof(unsigned), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     unsigned lines_bytes = 0;
     memcpy(&lines_bytes, s->h_u, sizeof(unsigned));

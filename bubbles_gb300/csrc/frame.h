@@ -13,18 +13,20 @@ constexpr int kFrameMass = 0x20;
 constexpr int kFrameSupported = kFramePosition | kFrameVelocity | kFrameDensity | kFrameMass;
 constexpr int kFrameLineCap = 128;   // "\t\t" + 8 numbers of at most 12 characters + separators
 
+constexpr int kFrameBlock = 128;     // lines of a block
+inline int frame_blocks(int n) { return (n + kFrameBlock - 1) / kFrameBlock; }
+
 struct FrameBufs {
     int capacity = 0;
-    char *lines = nullptr;        // capacity x kFrameLineCap
-    unsigned *lens = nullptr;     // capacity
-    unsigned *scan_in = nullptr;  // capacity
-    unsigned *offset = nullptr;   // capacity + 1
+    char *lines = nullptr;        // frame_blocks(capacity) x kFrameBlock x kFrameLineCap: staging
+    unsigned *lens = nullptr;     // frame_blocks(capacity): bytes of each block's lines
+    unsigned *offset = nullptr;   // frame_blocks(capacity) + 1
     unsigned *partials = nullptr;
     char *out = nullptr;          // capacity x kFrameLineCap
 };
 
 // Formats the particle lines of n particles (caller order through `slot`) and packs them
-// into F.out; F.offset[n] is the byte count.
+// into F.out; F.offset[frame_blocks(n)] is the byte count.
 void launch_frame_lines(int n, int flags, const float4 *pos, const float4 *vel, const float *rho,
                         const int *slot, float mass, FrameBufs &F, cudaStream_t s);
 

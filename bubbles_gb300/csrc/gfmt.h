@@ -5,18 +5,21 @@
 // (src/third/serializer.cpp:20-45): six significant digits, correctly rounded (ties to
 // even) from the exact binary value, then %e or %f style by the decimal exponent, trailing
 // zeros removed.  A float is m * 2^e with m < 2^24, so the six digits are
-// q = round(m * 2^e * 10^s) for s = 5 - X, X the decimal exponent.  q is computed exactly
-// as floor(A / B) with A = m * 2^max(e,0) * 10^max(s,0) and B = 2^max(-e,0) * 10^max(-s,0)
-// in 32-bit limbs (A < 2^192, B < 2^160), q (< 2^20) found bit by bit, and the remainder
-// decides the rounding.
+// q = round(m * 2^e * 10^s) for s = 5 - X, X the decimal exponent.  For e <= 0 and 0 <= s <= 19
+// (1e-14 up to 1e6) m * 10^s fits 128 bits and q is a shift of it, the bits shifted out
+// deciding the rounding.  Otherwise q is computed as floor(A / B) with
+// A = m * 2^max(e,0) * 10^max(s,0) and B = 2^max(-e,0) * 10^max(-s,0) in 32-bit limbs
+// (A < 2^192, B < 2^160), q (< 2^20) found bit by bit, and the remainder decides.
 #pragma once
 
 #include <stdint.h>
 
 #if defined(__CUDACC__)
 #define GFMT_FN __host__ __device__ __forceinline__
+#define GFMT_SLOW static __host__ __device__ __noinline__
 #else
 #define GFMT_FN inline
+#define GFMT_SLOW inline
 #endif
 
 namespace gfmt {
@@ -73,7 +76,7 @@ GFMT_FN void big_sub(Big &a, const Big &b) {   // a -= b (a >= b)
 
 // Six significant digits of m * 2^e at decimal exponent X: q = A / B rounded half to even.
 // Returns q (may be 10^6 after rounding up, or outside [10^5, 10^6) if X is wrong).
-GFMT_FN uint32_t digits6(uint32_t m, int e, int X) {
+GFMT_SLOW uint32_t digits6_big(uint32_t m, int e, int X) {
     const int s = 5 - X;
     Big A, B;
     big_set(A, m);
@@ -99,6 +102,21 @@ GFMT_FN uint32_t digits6(uint32_t m, int e, int X) {
     big_shl(r, 1);
     const int c = big_cmp(r, B);
     if (c > 0 || (c == 0 && (q & 1u))) q += 1;
+    return q;
+}
+
+GFMT_FN uint32_t digits6(uint32_t m, int e, int X) {
+    static constexpr uint64_t kTen[20] = {1ull, 10ull, 100ull, 1000ull, 10000ull, 100000ull, 1000000ull, 10000000ull,
+                                   100000000ull, 1000000000ull, 10000000000ull, 100000000000ull, 1000000000000ull,
+                                   10000000000000ull, 100000000000000ull, 1000000000000000ull, 10000000000000000ull,
+                                   100000000000000000ull, 1000000000000000000ull, 10000000000000000000ull};
+    const int s = 5 - X, r = -e;
+    if (r < 0 || r > 127 || s < 0 || s > 19) return digits6_big(m, e, X);
+    const unsigned __int128 v = (unsigned __int128)kTen[s] * m;   // < 2^88
+    const unsigned __int128 whole = v >> r, rest = v - (whole << r);
+    const unsigned __int128 half = r ? (unsigned __int128)1 << (r - 1) : 0;
+    uint32_t q = (uint32_t)whole;   // < 2^24: X is the decimal exponent or one below
+    if (r && (rest > half || (rest == half && (q & 1u)))) q += 1;
     return q;
 }
 
@@ -144,8 +162,7 @@ GFMT_FN int format_g(float f, char *out) {
     // decimal exponent estimate from the binary one: log10(m 2^e) ~ (bits(m) - 1 + e) log10 2
     int msb = 31;
     while (!(m >> msb)) msb--;
-    int X = (int)((double)(msb + e) * 0.30102999566398120);
-    if ((double)(msb + e) * 0.30102999566398120 < (double)X) X--;   // floor for negatives
+    int X = ((msb + e) * 1233) >> 12;   // the floor, within one; corrected below
     uint32_t q = digits6(m, e, X);
     for (int guard = 0; guard < 4 && (q < 100000u || q >= 1000000u); guard++) {
         if (q >= 1000000u) {
