@@ -364,6 +364,142 @@ k_density_mask(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, uns
                   D.listed + D.self, D.listed);
 }
 
+// The fewest particles: G lanes for each instead of a thread, which is one long chain of dependent loads,
+// about 216 candidates deep, on an idle chip.  The density pass takes sixteen lanes or eight,
+// the force pass, whose 29 members are the shorter chain, eight or four: as many as keep the density pass
+// within one wave of 8 blocks of 128 on 152 SMs; past it the extra instructions of splitting a
+// particle cost more than the latency they hide (12,144 particles: 16 and 8 lanes 375 us for seven
+// SPH substeps, 8 and 4 lanes 340, a thread each 371; 16,384: 8 and 4 lanes 370, a thread each 375; 20,000:
+// no difference; 35,937, 4 lanes: 461 against 374).
+constexpr int kGroupThreads = 128;
+constexpr int kGroupMembers = kMaxList;   // a particle with more (itself counted) is walked by one lane
+constexpr int kGroup16 = 152 * 8 * kGroupThreads / 16;   // particles, up to
+constexpr int kGroup8 = 2 * kGroup16;
+
+// The density pass, G lanes per particle: the lanes take every G-th candidate of the particle's nine rows,
+// all tested in float, and put the members' kernel values in shared memory in row order, where one
+// lane adds them in that order: the sum of k_density_mask to the bit.  The block's particles
+// are finished by the lanes of one warp and their lists written a row at a time by the others.
+// Bound by latency: two to four rounds of loads, then the chain of additions.  1,287 particles: 16.3 -> 10.2 us
+// (a timing event on either side included); with the force pass's lanes a substep 33.6 -> 24.3 us, of
+// 16,384 particles 36.1 -> 33.9.
+template <int G>
+__global__ void __launch_bounds__(kGroupThreads, 8)
+k_density_group(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, unsigned *__restrict__ cell,
+                const unsigned *__restrict__ start, float *__restrict__ rho, float *__restrict__ inv_rho,
+                float *__restrict__ press, int *__restrict__ nbr, ListEntry *__restrict__ list,
+                int compute_pressure, StepState *st) {
+    constexpr int S = kGroupThreads / G;           // particles of a block
+    __shared__ unsigned row_end[9][S];   // candidates up to the end of the row
+    __shared__ unsigned row_off[9][S];   // slot of a candidate of the row less its number
+    __shared__ float term[kGroupMembers][S];
+    __shared__ ListEntry member[kGroupMembers][S];
+    __shared__ int found[S], itself[S];   // members (-1: walked); the particle itself one
+    constexpr unsigned full = 0xffffffffu, group = (1u << G) - 1u;
+    const int grp = threadIdx.x / G, lane = threadIdx.x & (G - 1);
+    const int shift = threadIdx.x & 31 & ~(G - 1);
+    const int i0 = blockIdx.x * S;
+    const bool live = i0 + grp < P.n;
+    const int i = live ? i0 + grp : P.n - 1;
+    const float4 pi = pos[i];
+    const unsigned cw = cell[i], c = cw & ~kWide;
+    const GridDev &g = P.g;
+    int cx, cy, cz;
+    cell_coords(g, c, cx, cy, cz);
+    // rows r = 3 (dz + 1) + dy + 1, G at a time
+    constexpr int R = (9 + G - 1) / G;
+    unsigned b[R], len[R], total = 0;
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+        const int r = lane + G * u, dz = r / 3 - 1, dy = r - 3 * (r / 3) - 1;
+        b[u] = len[u] = 0;
+        if (live && r < 9 && cy + dy >= 0 && cy + dy < g.ny && cz + dz >= 0 && cz + dz < g.nz) {
+            const unsigned row = c + (unsigned)(dy * g.nx) + (unsigned)(dz * g.nx * g.ny);
+            b[u] = __ldg(&start[row - (cx > 0 ? 1u : 0u)]);
+            len[u] = __ldg(&start[row + (cx + 1 < g.nx ? 2u : 1u)]) - b[u];
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+        unsigned end = len[u];
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+            const unsigned y = __shfl_up_sync(full, end, o, G);
+            if (lane >= o) end += y;
+        }
+        end += total;
+        if (lane + G * u < 9) {
+            row_end[lane + G * u][grp] = end;
+            row_off[lane + G * u][grp] = b[u] - (end - len[u]);
+        }
+        total = __shfl_sync(full, end, G - 1, G);
+    }
+    __syncwarp();
+    const int self = std_member(P, pi, pi, DensitySum::dist(pi, pi)) ? 1 : 0;
+    // (the loops run as long as the warp's longest group, with every lane in them)
+    const unsigned work = total <= kMaxCandidates ? total : 0u, longest = __reduce_max_sync(full, work);
+    int cnt = 0, r = 0;
+    unsigned rend = row_end[0][grp], roff = row_off[0][grp];
+    constexpr int NB = 8;
+    for (unsigned k0 = 0; k0 < longest; k0 += NB * G) {
+        unsigned j[NB];
+        bool mem[NB];
+        float4 p[NB];
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const unsigned k = k0 + u * G + lane;
+            mem[u] = k < work;
+            while (mem[u] && k >= rend) {
+                r++;
+                rend = row_end[r][grp];
+                roff = row_off[r][grp];
+            }
+            j[u] = mem[u] ? roff + k : (unsigned)i;
+            p[u] = __ldg(&pos[j[u]]);
+        }
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const float r2 = DensitySum::dist(pi, p[u]);
+            mem[u] = mem[u] && std_member(P, pi, p[u], r2);
+            const unsigned m = (__ballot_sync(full, mem[u]) >> shift) & group;
+            const int q = cnt + __popc(m & ((1u << lane) - 1u));   // members before this one
+            cnt += __popc(m);
+            if (mem[u] && q < kGroupMembers) {
+                const float x = __fmaf_rn(-r2, P.inv_h2, 1.f);
+                term[q][grp] = __fmul_rn(__fmul_rn(x, x), x);
+                // the list leaves the particle itself out
+                if (j[u] != (unsigned)i) member[q - (j[u] > (unsigned)i ? self : 0)][grp] = j[u];
+            }
+        }
+    }
+    if (lane == 0) {
+        found[grp] = !live ? 0 : total > kMaxCandidates || cnt > kGroupMembers ? -1 : cnt;
+        itself[grp] = self;
+    }
+    __syncthreads();
+    const int mine = threadIdx.x & (S - 1);
+    cnt = found[mine];
+    const int listed = cnt - itself[mine];
+    if (threadIdx.x >= 32) {   // the lists, rows of the block's particles together
+        for (int q = (threadIdx.x - 32) / S; q < listed; q += (kGroupThreads - 32) / S)
+            list[(size_t)q * P.n + i0 + mine] = member[q][mine];
+    } else if (threadIdx.x < S && i0 + mine < P.n) {
+        const float4 pm = pos[i0 + mine];
+        const unsigned cm = cell[i0 + mine];
+        DensitySum D(list + i0 + mine);
+        if (cnt < 0) {
+            density_walk(P, pos, start, cm & ~kWide, pm, (unsigned)(i0 + mine), st, D);
+        } else {
+#pragma unroll 8
+            for (int q = 0; q < cnt; q++) D.sum = __fadd_rn(D.sum, term[q][mine]);
+            D.listed = listed;
+            D.self = itself[mine];
+        }
+        density_store(P, pos, vel, cell, rho, inv_rho, press, nbr, compute_pressure, st, i0 + mine, pm, cm, D.sum,
+                      D.listed + D.self, D.listed);
+    }
+}
+
 // ComputeNonPressureForceFor (sph_equations3.cpp:80-110), optionally followed by the
 // k = 0 PredictVelocityAndPositionFor (pcisph_equations3.cpp:3-28).
 //   predict 0: forces only; 1: the reference's k = 0 prediction (p = 0, Fp = 0, x* from F);
@@ -907,6 +1043,47 @@ k_worklist(Params P, const StepState *st, int k, int tile) {
     }
 }
 
+// A member's terms in the SPH force pass.
+struct SphPair {
+    float dx, dy, dz, c;      // the pressure force's terms are (dx, dy, dz) * c
+    float dvx, dvy, dvz, w;   // the viscosity's (dvx, dvy, dvz) * w
+    bool near, apart;         // inside the kernels; and not coincident
+    __device__ __forceinline__ SphPair(const Params &P, float4 pi, float4 vi, float4 pj, float4 vj, float ai, float kg,
+                                       float kv) {
+        const float r2 = dist2(pi, pj);
+        const float inv_d = rsqrtf(r2);
+        const float d = r2 > 0.f ? r2 * inv_d : 0.f;   // coincident particles: distance 0
+        near = d - P.h <= -P.iz;
+        apart = d >= P.iz;
+        const float x = 1.f - d * P.inv_h;
+        c = kg * (ai + pj.w) * x * x * inv_d;
+        w = kv * x * vj.w;   // vj.w = 1 / rho_j
+        dx = pj.x - pi.x;
+        dy = pj.y - pi.y;
+        dz = pj.z - pi.z;
+        dvx = vj.x - vi.x;
+        dvy = vj.y - vi.y;
+        dvz = vj.z - vi.z;
+    }
+};
+
+// What the force passes add a member to: t the pressure force's sum, f the rest.
+struct SphForce {
+    v3 f, t;
+    __device__ __forceinline__ void add(const SphPair &a) {
+        if (a.near) {
+            if (a.apart) {
+                t.x = __fmaf_rn(a.dx, a.c, t.x);
+                t.y = __fmaf_rn(a.dy, a.c, t.y);
+                t.z = __fmaf_rn(a.dz, a.c, t.z);
+            }
+            f.x = __fmaf_rn(a.dvx, a.w, f.x);
+            f.y = __fmaf_rn(a.dvy, a.w, f.y);
+            f.z = __fmaf_rn(a.dvz, a.w, f.z);
+        }
+    }
+};
+
 // ComputeAllForcesFor (sph_equations3.cpp:184-278, extended = 0) in Jacobi order: the
 // reference integrates each particle inside the force loop (:277), racing with its
 // neighbours' reads; here all forces read the step-start state and the integrated
@@ -924,35 +1101,15 @@ k_sph_forces(Params P, const float4 *__restrict__ pos, const float4 *__restrict_
         const float4 pi = pos[i];
         const float4 vi = vel[i];
         const float ai = pi.w;   // p_i / rho_i^2
-        float fx = P.mass * P.gx - P.drag * vi.x;
-        float fy = P.mass * P.gy - P.drag * vi.y;
-        float fz = P.mass * P.gz - P.drag * vi.z;
-        float tx = 0.f, ty = 0.f, tz = 0.f;
+        SphForce a{V(P.mass * P.gx - P.drag * vi.x, P.mass * P.gy - P.drag * vi.y, P.mass * P.gz - P.drag * vi.z),
+                   V(0.f, 0.f, 0.f)};
         const float kg = P.m2 * P.spiky_dw_c;
         const float kv = P.visc_m2 * P.spiky_d2w_c;
         tile_members<NB>(
             P, start, list, nbr, pos, cell[i], i,
             [&](unsigned j) { return PosVel{__ldg(&pos[j]), __ldg(&vel[j])}; },
-            [&](const PosVel &nb) {
-                const float4 pj = nb.p, vj = nb.v;   // vj.w = 1 / rho_j
-                const float r2 = dist2(pi, pj);
-                const float inv_d = rsqrtf(r2);
-                const float d = r2 > 0.f ? r2 * inv_d : 0.f;   // coincident particles: distance 0
-                if (d - P.h <= -P.iz) {
-                    const float x = 1.f - d * P.inv_h;
-                    if (d >= P.iz) {
-                        const float c = kg * (ai + pj.w) * x * x * inv_d;
-                        tx += (pj.x - pi.x) * c;
-                        ty += (pj.y - pi.y) * c;
-                        tz += (pj.z - pi.z) * c;
-                    }
-                    const float w = kv * x * vj.w;
-                    fx += (vj.x - vi.x) * w;
-                    fy += (vj.y - vi.y) * w;
-                    fz += (vj.z - vi.z) * w;
-                }
-            });
-        const v3 f = V(fx - tx, fy - ty, fz - tz);
+            [&](const PosVel &nb) { a.add(SphPair(P, pi, vi, nb.p, nb.v, ai, kg, kv)); });
+        const v3 f = V(a.f.x - a.t.x, a.f.y - a.t.y, a.f.z - a.t.z);
         force[i] = F4(f);
         v3 x = V(pi), v = V(vi);
         integrate_particle(P, dt, f, &x, &v);
@@ -963,6 +1120,118 @@ k_sph_forces(Params P, const float4 *__restrict__ pos, const float4 *__restrict_
     }
     fbits = warp_max_u(fbits);
     if ((threadIdx.x & 31) == 0 && fbits) atomicMax(&st->max_force_bits, fbits);
+    count_nonfinite(bad, st);
+}
+
+// The same with G lanes per particle (see kGroup16): the lanes take every G-th member and leave its
+// terms in shared memory, 4 G members at a time, and each of the six sums is added up over them in
+// list order by a lane, as k_sph_forces adds them.  One warp then integrates the block's particles.  Blocks
+// of 16 KB and 64 registers: with all 64 members' terms in shared memory, 6 blocks an SM, 16,384
+// particles took 18 us, so 14 (four lanes 12).  1,287 particles: 12.3 -> 8.2 us.
+template <int G>
+__global__ void __launch_bounds__(kGroupThreads, 8)
+k_sph_forces_group(Params P, const float4 *__restrict__ pos, const float4 *__restrict__ vel,
+                   const unsigned *__restrict__ cell, const unsigned *__restrict__ start,
+                   const ListEntry *__restrict__ list, const int *__restrict__ nbr, float4 *__restrict__ force,
+                   float4 *__restrict__ pos_out, float4 *__restrict__ vel_out, StepState *st, float dt) {
+    constexpr int S = kGroupThreads / G;   // particles of a block
+    constexpr int NB = 4, kGroupTerms = NB * G;
+    __shared__ float4 term[2][kGroupTerms][S];   // (dx, dy, dz, c), (dvx, dvy, dvz, w)
+    __shared__ float sums[6][S];
+    constexpr unsigned full = 0xffffffffu, group = (1u << G) - 1u;
+    const int grp = threadIdx.x / G, lane = threadIdx.x & (G - 1);
+    const int shift = threadIdx.x & 31 & ~(G - 1);
+    const bool live = blockIdx.x * S + grp < P.n;
+    const int i = live ? blockIdx.x * S + grp : P.n - 1;
+    const float4 pi = pos[i];
+    const float4 vi = vel[i];
+    const float ai = pi.w;
+    const v3 f0 = V(P.mass * P.gx - P.drag * vi.x, P.mass * P.gy - P.drag * vi.y, P.mass * P.gz - P.drag * vi.z);
+    const float kg = P.m2 * P.spiky_dw_c;
+    const float kv = P.visc_m2 * P.spiky_d2w_c;
+    const unsigned cw = cell[i];
+    const bool wide = (cw & kWide) != 0;
+    const int cnt = live && !wide ? __ldg(&nbr[i]) - 1 : 0;
+    const int longest = __reduce_max_sync(full, cnt);
+    const ListEntry *const l = list + i;
+    // the six sums: with eight lanes t in lanes 0 .. 2 and f in 3 .. 5, with four both in 0 .. 2
+    // (the lanes left over along with the last)
+    constexpr int per = G >= 6 ? 1 : 2;
+    const int k = per == 2 ? min(lane, 2) : lane < 3 ? lane : min(lane, 5) - 3;
+    const bool is_f = per == 1 && lane >= 3;
+    const float fk = k == 0 ? f0.x : k == 1 ? f0.y : f0.z;
+    float acc[per];
+    acc[0] = is_f ? fk : 0.f;
+    if (per == 2) acc[per - 1] = fk;
+    const float *const e0 = reinterpret_cast<const float *>(&term[is_f ? 1 : 0][0][grp]);
+    for (int q0 = 0; q0 < longest; q0 += kGroupTerms) {
+        unsigned j[NB];
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const int q = q0 + u * G + lane;
+            j[u] = q < cnt ? __ldg(l + (size_t)q * P.n) : (unsigned)i;
+        }
+        PosVel nb[NB];
+#pragma unroll
+        for (int u = 0; u < NB; u++) nb[u] = PosVel{__ldg(&pos[j[u]]), __ldg(&vel[j[u]])};
+        unsigned near = 0, apart = 0;   // the group's members with terms
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const int q = u * G + lane;
+            const SphPair a(P, pi, vi, nb[u].p, nb[u].v, ai, kg, kv);
+            const bool in = q0 + q < cnt && a.near;
+            if (in) {
+                term[0][q][grp] = make_float4(a.dx, a.dy, a.dz, a.c);
+                term[1][q][grp] = make_float4(a.dvx, a.dvy, a.dvz, a.w);
+            }
+            near |= ((__ballot_sync(full, in) >> shift) & group) << (u * G);
+            apart |= ((__ballot_sync(full, in && a.apart) >> shift) & group) << (u * G);
+        }
+        __syncwarp();
+        const unsigned take = is_f ? near : apart;
+        const float *e = e0;
+        const int some = min(cnt - q0, kGroupTerms);
+#pragma unroll 4
+        for (int q = 0; q < some; q++, e += 4 * S) {
+            if ((take >> q) & 1u) acc[0] = __fmaf_rn(e[k], e[3], acc[0]);
+            if (per == 2 && ((near >> q) & 1u))
+                acc[per - 1] = __fmaf_rn(e[4 * kGroupTerms * S + k], e[4 * kGroupTerms * S + 3], acc[per - 1]);
+        }
+        __syncwarp();
+    }
+    if (per == 1 ? lane < 6 : lane < 3) {
+        sums[lane][grp] = acc[0];
+        if (per == 2) sums[3 + lane][grp] = acc[per - 1];
+    }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    // the first warp: a lane per particle
+    const int at = blockIdx.x * S + threadIdx.x;
+    unsigned fbits = 0;
+    bool bad = false;
+    if (threadIdx.x < S && at < P.n) {
+        const float4 pm = pos[at], vm = vel[at];
+        const unsigned cm = cell[at];
+        const int t = threadIdx.x;
+        v3 f = V(sums[3][t] - sums[0][t], sums[4][t] - sums[1][t], sums[5][t] - sums[2][t]);
+        if (cm & kWide) {
+            SphForce a{V(P.mass * P.gx - P.drag * vm.x, P.mass * P.gy - P.drag * vm.y, P.mass * P.gz - P.drag * vm.z),
+                       V(0.f, 0.f, 0.f)};
+            tile_members<1>(P, start, list, nbr, pos, cm, at,
+                            [&](unsigned j) { return PosVel{__ldg(&pos[j]), __ldg(&vel[j])}; },
+                            [&](const PosVel &nb) { a.add(SphPair(P, pm, vm, nb.p, nb.v, pm.w, kg, kv)); });
+            f = V(a.f.x - a.t.x, a.f.y - a.t.y, a.f.z - a.t.z);
+        }
+        force[at] = F4(f);
+        v3 x = V(pm), v = V(vm);
+        integrate_particle(P, dt, f, &x, &v);
+        pos_out[at] = F4(x);
+        vel_out[at] = F4(v);
+        fbits = __float_as_uint(vlen(f));
+        bad = !finite_state(x, v);
+    }
+    fbits = warp_max_u(fbits);
+    if (threadIdx.x == 0 && fbits) atomicMax(&st->max_force_bits, fbits);
     count_nonfinite(bad, st);
 }
 
@@ -1075,13 +1344,24 @@ void launch_export_members(const Params &P, const DevBufs &B, int buf, int pid_b
 void launch_density(const Params &P, const DevBufs &B, int buf, int compute_pressure, cudaStream_t s, bool recorded) {
     BBG_PBEGIN(B, KID_DENSITY, s, -1);
     const int t = B.tune.block;
-    if (!recorded)
-        k_filter_records<<<blocks_for(P.n, kThreads), kThreads, 0, s>>>(P, B.pos[buf], B.cell,
-                                                                        reinterpret_cast<__half *>(B.frec));
-    const auto density = P.n <= kFew ? k_density_mask<true> : k_density_mask<false>;
-    density<<<blocks_for(P.n, t), t, sizeof(uint2) * kMasks * (size_t)t, s>>>(
-        P, B.pos[buf], B.vel[buf], B.cell, B.start, B.frec, B.rho, B.inv_rho, B.press, B.nbr, B.list,
-        compute_pressure, B.st);
+#define DENSITY_GROUP(G)                                                                          \
+    k_density_group<G><<<blocks_for(P.n, kGroupThreads / G), kGroupThreads, 0, s>>>(              \
+        P, B.pos[buf], B.vel[buf], B.cell, B.start, B.rho, B.inv_rho, B.press, B.nbr, B.list,     \
+        compute_pressure, B.st)
+    if (P.n <= kGroup16) {
+        DENSITY_GROUP(16);
+    } else if (P.n <= kGroup8) {
+        DENSITY_GROUP(8);
+    } else {
+        if (!recorded)
+            k_filter_records<<<blocks_for(P.n, kThreads), kThreads, 0, s>>>(P, B.pos[buf], B.cell,
+                                                                            reinterpret_cast<__half *>(B.frec));
+        const auto density = P.n <= kFew ? k_density_mask<true> : k_density_mask<false>;
+        density<<<blocks_for(P.n, t), t, sizeof(uint2) * kMasks * (size_t)t, s>>>(
+            P, B.pos[buf], B.vel[buf], B.cell, B.start, B.frec, B.rho, B.inv_rho, B.press, B.nbr, B.list,
+            compute_pressure, B.st);
+    }
+#undef DENSITY_GROUP
     if (P.nscenes > 0 && P.n > 0) {
         // batch: each scene's slot range (the scene of every slot was set just above)
         cudaMemsetAsync(P.scene_first, 0x7f, sizeof(int) * (size_t)P.nscenes, s);
@@ -1274,8 +1554,12 @@ void launch_pressure_force(const Params &P, const DevBufs &B, int buf, int k, in
 
 void launch_sph_forces(const Params &P, const DevBufs &B, int buf, float dt, cudaStream_t s) {
     BBG_PBEGIN(B, KID_SPH_FORCES, s, -1);
-    const auto forces = P.n <= kFew ? k_sph_forces<kFewBatchPosVel> : k_sph_forces<(kGatherBatch < 4 ? kGatherBatch : 4)>;
-    forces<<<blocks_for(P.n, B.tune.block), B.tune.block, 0, s>>>(
+    const int lanes = P.n <= kGroup16 ? 8 : P.n <= kGroup8 ? 4 : 1, t = lanes > 1 ? kGroupThreads : B.tune.block;
+    const auto forces = lanes == 8    ? k_sph_forces_group<8>
+                        : lanes == 4  ? k_sph_forces_group<4>
+                        : P.n <= kFew ? k_sph_forces<kFewBatchPosVel>
+                                      : k_sph_forces<(kGatherBatch < 4 ? kGatherBatch : 4)>;
+    forces<<<blocks_for(P.n, t / lanes), t, 0, s>>>(
         P, B.pos[buf], B.vel[buf], B.cell, B.start, B.list, B.nbr, B.force, B.pos[1 - buf],
         B.vel[1 - buf], B.st, dt);
     BBG_PEND(B, s);
