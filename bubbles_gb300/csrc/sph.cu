@@ -621,6 +621,35 @@ __global__ void k_pack_acoef(int n, float4 *pos, const float *__restrict__ press
     reinterpret_cast<float *>(&pos[i])[3] = press[i] / (d * d);
 }
 
+// The end of PredictPressureFor (pcisph_equations3.cpp:60-90) for particle i, from the kernel sum at
+// predicted positions: density, its error, pressure and p / rho*^2.  Returns |err|.
+__device__ __forceinline__ float pred_density_end(const Params &P, float4 *pos, float *__restrict__ press,
+                                                  float *__restrict__ rhostar, float *__restrict__ derr, float delta,
+                                                  int clamp_total, int i, float sum) {
+    const float density = sum * P.std_c * P.mass;
+    float err = density - P.target_density;
+    float pr = delta * err;
+    float p;
+    if (clamp_total) {
+        // warm-started corrector: the increment may be negative, the total is scaled
+        // like a negative pressure, so an overestimated start can be corrected
+        if (err < 0.f) err *= P.neg_scale;
+        p = press[i] + pr;
+        if (p < 0.f) p *= P.neg_scale;
+    } else {
+        if (pr < 0.f) {
+            pr *= P.neg_scale;
+            err *= P.neg_scale;
+        }
+        p = press[i] + pr;
+    }
+    press[i] = p;
+    rhostar[i] = density;
+    derr[i] = err;
+    reinterpret_cast<float *>(&pos[i])[3] = p / (density * density);   // pos.w = p / rho*^2
+    return fabsf(err);
+}
+
 // PredictPressureFor (pcisph_equations3.cpp:60-90) of particle i over the step-start
 // neighbour set at predicted positions, with the density error stored (tolerance mode);
 // also p / rho*^2 for the pressure force.  Returns |err| (0 for a particle not updated)
@@ -651,28 +680,7 @@ __device__ __forceinline__ float pred_density_one(const Params &P, float4 *pos, 
                     sum += x * x * x;
                 }
             });
-        const float density = sum * P.std_c * P.mass;
-        float err = density - P.target_density;
-        float pr = delta * err;
-        float p;
-        if (clamp_total) {
-            // warm-started corrector: the increment may be negative, the total is scaled
-            // like a negative pressure, so an overestimated start can be corrected
-            if (err < 0.f) err *= P.neg_scale;
-            p = press[i] + pr;
-            if (p < 0.f) p *= P.neg_scale;
-        } else {
-            if (pr < 0.f) {
-                pr *= P.neg_scale;
-                err *= P.neg_scale;
-            }
-            p = press[i] + pr;
-        }
-        press[i] = p;
-        rhostar[i] = density;
-        derr[i] = err;
-        reinterpret_cast<float *>(&pos[i])[3] = p / (density * density);   // pos.w = p / rho*^2
-        aerr = fabsf(err);
+        aerr = pred_density_end(P, pos, press, rhostar, derr, delta, clamp_total, i, sum);
     }
     return aerr;
 }
@@ -839,6 +847,31 @@ k_pred_density_wl(Params P, float4 *pos, const float4 *__restrict__ xstar,
     error_reduce(st, amax, asum, k);
 }
 
+// What follows a particle's pressure force fp: the next prediction, or with `last`
+// AccumulateForcesFor + TimeIntegrationFor.
+__device__ __forceinline__ void pressure_force_end(const Params &P, const float4 *__restrict__ vel, float4 *__restrict__ force,
+                                                   float4 *__restrict__ pforce, float4 *__restrict__ xstar,
+                                                   float4 *__restrict__ pos_out, float4 *__restrict__ vel_out, float dt,
+                                                   float dt_over_m, int mode, bool last, int i, float4 pi, v3 fp,
+                                                   unsigned &fbits, bool &bad) {
+    pforce[i] = F4(fp);
+    const v3 f = V(force[i]);
+    if (last) {
+        const v3 ft = vadd(f, fp);
+        force[i] = F4(ft);
+        v3 x = V(pi), v = V(vel[i]);
+        integrate_particle(P, dt, ft, &x, &v);
+        pos_out[i] = F4(x);
+        vel_out[i] = F4(v);
+        fbits = max(fbits, __float_as_uint(vlen(ft)));
+        bad = bad || !finite_state(x, v);
+    } else if (mode != 1) {
+        v3 xs;
+        predict_particle(P, dt, dt_over_m, f, fp, V(pi), V(vel[i]), &xs);
+        xstar[i] = F4(xs);
+    }
+}
+
 // PredictPressureForceFor (pcisph_equations3.cpp:114-155) of particle i at the current
 // positions, then either the next prediction or AccumulateForcesFor + TimeIntegrationFor.
 // `last`: iteration k ends the corrector (single scene); batches decide per scene.
@@ -881,23 +914,8 @@ __device__ __forceinline__ void pressure_force_one(const Params &P, const float4
                 tz += (pj.z - pi.z) * c;
             }
         });
-    const v3 fp = V(-tx, -ty, -tz);
-    pforce[i] = F4(fp);
-    const v3 f = V(force[i]);
-    if (last) {
-        const v3 ft = vadd(f, fp);
-        force[i] = F4(ft);
-        v3 x = V(pi), v = V(vel[i]);
-        integrate_particle(P, dt, ft, &x, &v);
-        pos_out[i] = F4(x);
-        vel_out[i] = F4(v);
-        fbits = max(fbits, __float_as_uint(vlen(ft)));
-        bad = bad || !finite_state(x, v);
-    } else if (mode != 1) {
-        v3 xs;
-        predict_particle(P, dt, dt_over_m, f, fp, V(pi), V(vel[i]), &xs);
-        xstar[i] = F4(xs);
-    }
+    pressure_force_end(P, vel, force, pforce, xstar, pos_out, vel_out, dt, dt_over_m, mode, last, i, pi,
+                       V(-tx, -ty, -tz), fbits, bad);
 }
 
 __device__ __forceinline__ bool corrector_ends(const Params &P, const StepState *st, int k, int max_it, int mode) {
@@ -1041,6 +1059,142 @@ k_worklist(Params P, const StepState *st, int k, int tile) {
         P.wl_ctr[0] = 0;
         P.wl_ctr[1] = 0;
     }
+}
+
+// The corrector's passes with G lanes per particle (see kGroup16), in the manner of
+// k_sph_forces_group; single scenes only, since a batch's blocks walk tiles of its scenes.  A
+// substep of 8,400 particles, 3 iterations: 98.7 -> 92.1 us; 12,144, 9 iterations: 201 -> 189; 18,252, 5
+// iterations: 137 -> 133.  What is left of an iteration is two launches and the loop's condition.
+template <int G>
+__global__ void __launch_bounds__(kGroupThreads, 8)
+k_pred_density_group(Params P, float4 *pos, const float4 *__restrict__ xstar, const unsigned *__restrict__ cell,
+                     const unsigned *__restrict__ start, const ListEntry *__restrict__ list,
+                     const int *__restrict__ nbr, float *__restrict__ press, float *__restrict__ rhostar,
+                     float *__restrict__ derr, StepState *st, int k, float delta, int clamp_total) {
+    if (!density_iteration(P, st, k)) return;
+    constexpr int S = kGroupThreads / G, NB = 32 / G;
+    __shared__ float term[kMaxList][S];   // x of the member's x^3; 0 outside the kernel, which adds nothing
+    const int grp = threadIdx.x / G, lane = threadIdx.x & (G - 1);
+    const int at = blockIdx.x * S + grp;
+    if (at < P.n) {
+        const float4 xi = xstar[at];
+        const unsigned cw = cell[at];
+        const int cnt = cw & kWide ? 0 : __ldg(&nbr[at]) - 1;
+        const ListEntry *const l = list + at;
+        for (int q0 = lane; q0 < cnt; q0 += NB * G) {
+            unsigned j[NB];
+#pragma unroll
+            for (int u = 0; u < NB; u++) j[u] = q0 + u * G < cnt ? __ldg(l + (size_t)(q0 + u * G) * P.n) : (unsigned)at;
+            float4 xj[NB];
+#pragma unroll
+            for (int u = 0; u < NB; u++) xj[u] = __ldg(&xstar[j[u]]);
+#pragma unroll
+            for (int u = 0; u < NB; u++) {
+                const float r2 = dist2(xi, xj[u]);
+                if (q0 + u * G < cnt) term[q0 + u * G][grp] = r2 < P.h2mz ? __fmaf_rn(-r2, P.inv_h2, 1.f) : 0.f;
+            }
+        }
+    }
+    __syncthreads();
+    float aerr = 0.f;
+    const int i = blockIdx.x * S + threadIdx.x;
+    if (threadIdx.x < S && i < P.n) {
+        const unsigned cw = cell[i];
+        float sum = 1.f;   // the particle itself
+        if (cw & kWide) {
+            const float4 xi = xstar[i];
+            tile_members<1>(P, start, list, nbr, pos, cw, i, [&](unsigned j) { return __ldg(&xstar[j]); },
+                            [&](const float4 xj) {
+                                const float r2 = dist2(xi, xj);
+                                if (r2 < P.h2mz) {
+                                    const float x = __fmaf_rn(-r2, P.inv_h2, 1.f);
+                                    sum = __fmaf_rn(__fmul_rn(x, x), x, sum);
+                                }
+                            });
+        } else {
+            const int cnt = __ldg(&nbr[i]) - 1;
+#pragma unroll 8
+            for (int q = 0; q < cnt; q++) {
+                const float x = term[q][threadIdx.x];
+                sum = __fmaf_rn(__fmul_rn(x, x), x, sum);
+            }
+        }
+        aerr = pred_density_end(P, pos, press, rhostar, derr, delta, clamp_total, i, sum);
+    }
+    error_reduce(st, aerr, aerr, k);
+}
+
+template <int G>
+__global__ void __launch_bounds__(kGroupThreads, 8)
+k_pressure_force_group(Params P, const float4 *__restrict__ pos, const float4 *__restrict__ vel,
+                       const unsigned *__restrict__ cell, const unsigned *__restrict__ start,
+                       const ListEntry *__restrict__ list, const int *__restrict__ nbr, float4 *__restrict__ force,
+                       float4 *__restrict__ pforce, float4 *__restrict__ xstar, float4 *__restrict__ pos_out,
+                       float4 *__restrict__ vel_out, StepState *st, int k, int max_it, float dt, float dt_over_m,
+                       int mode, cudaGraphConditionalHandle loop) {
+    if (!force_iteration(P, st, k, max_it, loop)) return;
+    const bool last = corrector_ends(P, st, k, max_it, mode);
+    constexpr int S = kGroupThreads / G, NB = G == 4 ? 4 : 32 / G, kTerms = NB * G;
+    __shared__ float4 term[kTerms][S];   // (dx, dy, dz, c): the member adds (dx, dy, dz) * c; (0, 0, 0, 0): nothing
+    __shared__ float sums[3][S];
+    const int grp = threadIdx.x / G, lane = threadIdx.x & (G - 1);
+    const int at = blockIdx.x * S + grp;
+    const bool live = at < P.n;
+    const float4 pa = pos[live ? at : P.n - 1];
+    const unsigned ca = cell[live ? at : P.n - 1];
+    const int cnt = live && !(ca & kWide) ? __ldg(&nbr[at]) - 1 : 0;
+    const int longest = __reduce_max_sync(0xffffffffu, cnt);
+    const ListEntry *const l = list + (live ? at : 0);
+    const float kg = P.m2 * P.spiky_dw_c;
+    const int dim = min(lane, 2);
+    float acc = 0.f;
+    for (int q0 = 0; q0 < longest; q0 += kTerms) {
+        unsigned j[NB];
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const int q = q0 + u * G + lane;
+            j[u] = q < cnt ? __ldg(l + (size_t)q * P.n) : 0u;
+        }
+        float4 pj[NB];
+#pragma unroll
+        for (int u = 0; u < NB; u++) pj[u] = __ldg(&pos[j[u]]);
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+            const float r2 = dist2(pa, pj[u]);
+            const float inv_d = rsqrtf(r2);
+            const float d = r2 > 0.f ? r2 * inv_d : 0.f;   // coincident particles: distance 0
+            const float x = 1.f - d * P.inv_h;
+            const float c = kg * (pa.w + pj[u].w) * x * x * inv_d;
+            const bool in = d - P.h <= -P.iz && d >= P.iz;
+            term[u * G + lane][grp] = in ? make_float4(pj[u].x - pa.x, pj[u].y - pa.y, pj[u].z - pa.z, c)
+                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncwarp();
+        const float *e = reinterpret_cast<const float *>(&term[0][grp]);
+        const int some = min(cnt - q0, kTerms);
+#pragma unroll 8
+        for (int q = 0; q < some; q++, e += 4 * S) acc = __fmaf_rn(e[dim], e[3], acc);
+        __syncwarp();
+    }
+    if (lane < 3) sums[lane][grp] = acc;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const int i = blockIdx.x * S + threadIdx.x;
+    unsigned fbits = 0;
+    bool bad = false;
+    if (threadIdx.x < S && i < P.n) {
+        if (cell[i] & kWide) {
+            pressure_force_one<1>(P, pos, vel, cell, start, list, nbr, force, pforce, xstar, pos_out, vel_out, k, max_it,
+                                  dt, dt_over_m, mode, last, i, fbits, bad);
+        } else {
+            const v3 fp = V(-sums[0][threadIdx.x], -sums[1][threadIdx.x], -sums[2][threadIdx.x]);
+            pressure_force_end(P, vel, force, pforce, xstar, pos_out, vel_out, dt, dt_over_m, mode, last, i, pos[i], fp,
+                               fbits, bad);
+        }
+    }
+    fbits = warp_max_u(fbits);
+    if (threadIdx.x == 0 && fbits) atomicMax(&st->max_force_bits, fbits);
+    count_nonfinite(bad, st);
 }
 
 // A member's terms in the SPH force pass.
@@ -1487,7 +1641,14 @@ void launch_pred_density(const Params &P, const DevBufs &B, int buf, int k, floa
 #define PD_LAUNCH(...)                                                                            \
     k_pred_density<__VA_ARGS__><<<grid, t, 0, s>>>(Q, B.pos[buf], B.xstar, B.cell, B.start, B.list, B.nbr, \
                                                B.press, B.rhostar, B.derr, B.st, k, delta, clamp_total, wl)
-        if (P.n <= kFew) PD_LAUNCH(kFewBatch, 1, 1);
+#define PD_GROUP(G)                                                                                       \
+    k_pred_density_group<G><<<blocks_for(P.n, kGroupThreads / G), kGroupThreads, 0, s>>>(                  \
+        P, B.pos[buf], B.xstar, B.cell, B.start, B.list, B.nbr, B.press, B.rhostar, B.derr, B.st, k, delta, \
+        clamp_total)
+        if (P.n <= kGroup16 && P.nscenes == 0) PD_GROUP(8);
+        else if (P.n <= kGroup8 && P.nscenes == 0) PD_GROUP(4);
+        else if (P.n <= kFew) PD_LAUNCH(kFewBatch, 1, 1);
+#undef PD_GROUP
         else switch (B.tune.batch_pd * 10 + ppt) {
             case 21: PD_LAUNCH(2, 1); break;
             case 81: PD_LAUNCH(8, 1); break;
@@ -1538,7 +1699,14 @@ void launch_pressure_force(const Params &P, const DevBufs &B, int buf, int k, in
     k_pressure_force<__VA_ARGS__><<<grid, t, 0, s>>>(                                                       \
         Q, B.pos[buf], B.vel[buf], B.cell, B.start, B.list, B.nbr, B.force, B.pforce, B.xstar,           \
         B.pos[1 - buf], B.vel[1 - buf], B.st, k, max_it, dt, dt_over_m, mode, wl, loop)
-        if (P.n <= kFew) PF_LAUNCH(kFewBatch, 1, 1);
+#define PF_GROUP(G)                                                                                      \
+    k_pressure_force_group<G><<<blocks_for(P.n, kGroupThreads / G), kGroupThreads, 0, s>>>(                \
+        P, B.pos[buf], B.vel[buf], B.cell, B.start, B.list, B.nbr, B.force, B.pforce, B.xstar,             \
+        B.pos[1 - buf], B.vel[1 - buf], B.st, k, max_it, dt, dt_over_m, mode, loop)
+        if (P.n <= kGroup16 && P.nscenes == 0) PF_GROUP(8);
+        else if (P.n <= kGroup8 && P.nscenes == 0) PF_GROUP(4);
+        else if (P.n <= kFew) PF_LAUNCH(kFewBatch, 1, 1);
+#undef PF_GROUP
         else switch (B.tune.batch_pf * 10 + ppt) {
             case 21: PF_LAUNCH(2, 1); break;
             case 81: PF_LAUNCH(8, 1); break;

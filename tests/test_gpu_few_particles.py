@@ -50,3 +50,28 @@ def test_same_bits_as_the_general_passes(gpu, name):
         out.append([np.asarray(a)[:n].copy() for a in (count, lists, rho, force, x, u)])
     for what, a, b in zip(("counts", "lists", "density", "force", "positions", "velocities"), *out):
         assert a.tobytes() == b.tobytes(), what
+
+
+@pytest.mark.parametrize("name", ["one", "three", "lattice", "dense", "crowd", "twins", "walls", "last16", "first8",
+                                  "last8"])
+def test_same_bits_of_the_corrector(gpu, name):
+    import bubbles_gb300 as bb
+    from bubbles_gb300 import scenes
+    few = states()[name].astype(np.float32)
+    n = len(few)
+    vel = np.random.default_rng(6).normal(0, 0.3, (n, 3)).astype(np.float32)
+    out = []
+    for pos, v in ((few, vel), (np.concatenate([few, FILL]), np.concatenate([vel, np.zeros_like(FILL)]))):
+        sc = scenes.base_scene("pcisph", 0.02, (2.4, 0.6, 0.7))
+        sc["pcisph_mode"] = "tolerance"
+        sc["max_iterations"] = 4
+        sc["max_density_error_ratio"] = 1e-12   # never met: both run all iterations
+        with bb.Solver(sc, pos=pos, vel=v) as s:
+            s.update_grid_distribution()
+            s.advance_time_step(1e-4)
+            fields = [s.get(f) for f in (bb.FIELD_DENSITY, bb.FIELD_PRESSURE, bb.FIELD_PRED_DENSITY,
+                                         bb.FIELD_DENSITY_ERROR, bb.FIELD_PRESSURE_FORCE, bb.FIELD_FORCE)]
+            fields += list(s.download())
+        out.append([np.asarray(a)[:n].copy() for a in fields])
+    for k, (a, b) in enumerate(zip(*out)):
+        assert a.tobytes() == b.tobytes(), k
