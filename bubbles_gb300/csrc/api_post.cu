@@ -568,6 +568,7 @@ bbg_status bbg_particle_sdf(bbg_solver s, int method, double kernel_radius, doub
     const float dx = A.g.bmax[0] - A.g.bmin[0], dy = A.g.bmax[1] - A.g.bmin[1], dz = A.g.bmax[2] - A.g.bmin[2];
     A.inf = std::sqrt(dx * dx + dy * dy + dz * dz);
     A.radius = (float)kernel_radius;
+    A.near2 = largest_square(std::nextafter(A.radius, 0.f));
     A.offset = A.radius * 0.25f;
     A.mass = s->mass;
     A.r2 = A.radius * A.radius;

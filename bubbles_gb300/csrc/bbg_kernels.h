@@ -175,6 +175,7 @@ struct SurfaceArgs {
     float org[3], sp[3];
     float inf;            // the domain grid's diagonal length
     float radius;         // kernel radius
+    float near2;          // the largest square whose rounded root is below it
     float offset;         // Zhu-Bridson: radius x threshold
     float mass, r2;       // SPH: particle mass, radius squared,
     double wc;            // 315 / (64 pi radius^3)

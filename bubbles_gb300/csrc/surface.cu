@@ -7,6 +7,12 @@
 // operation is explicitly rounded in the reference's order; the steps the reference takes
 // in double (the cubic weight of Zhu-Bridson, the std kernel's constant) give the double's result
 // (double_cube): 262,144 particles, 111 -> 70 us.
+//
+// A node's candidates (216 in a full block) are tested four at a time, by squared distance against
+// the largest square whose root is below the radius, and the slots of those that count kept in shared
+// memory in walk order; the weights then run over them alone.  With the weight in the walk, one
+// load at a time and half the lanes idle, the pass waited for its loads at 38 % of the issue slots: 68 -> 45 us
+// (129,168 nodes).  Blocks of 64, since most nodes of a field lie outside the fluid and end at once.
 #include "bbg_internal.cuh"
 #include "bbg_kernels.h"
 
@@ -19,7 +25,12 @@ __device__ __forceinline__ float dist3(v3 a, float4 b) {
     return __fsqrt_rn(fa(fa(fm(ex, ex), fm(ey, ey)), fm(ez, ez)));
 }
 
-__global__ void k_particle_sdf(SurfaceArgs A, float *__restrict__ out) {
+constexpr int kFieldThreads = 64, kFieldSlots = 64;   // slots kept before they are summed
+
+__global__ void __launch_bounds__(kFieldThreads)
+k_particle_sdf(SurfaceArgs A, float *__restrict__ out) {
+    __shared__ unsigned near[kFieldSlots][kFieldThreads];
+    const int t = threadIdx.x;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long total = (long long)A.nodes[0] * A.nodes[1] * A.nodes[2];
     if (i >= total) return;
@@ -40,36 +51,74 @@ __global__ void k_particle_sdf(SurfaceArgs A, float *__restrict__ out) {
     const int cz = (int)(c / ((unsigned)g.nx * (unsigned)g.ny));
     const float R = A.radius;
     float wsum = 0.f, ax = 0.f, ay = 0.f, az = 0.f;
-    for (int y = max(cy - 1, 0); y <= min(cy + 1, g.ny - 1); y++)
-        for (int x = max(cx - 1, 0); x <= min(cx + 1, g.nx - 1); x++)
-            for (int z = max(cz - 1, 0); z <= min(cz + 1, g.nz - 1); z++) {
-                const unsigned nb = (unsigned)x + (unsigned)y * g.nx + (unsigned)z * g.nx * g.ny;
-                for (unsigned s = A.start[nb]; s < A.start[nb + 1]; s++) {
-                    const float4 xi = A.pos[s];
-                    const float d = dist3(p, xi);
-                    if (A.method == 0) {
-                        // ZhuBridsonSDF: k_cub(|p - x| / R) = Max(0, (1 - s^2)^3), the cube in double
-                        if (d < R) {
-                            const float t = fdv(d, R);
-                            const float cub = double_cube_1m(fm(t, t));
-                            const float w = 0.f < cub ? cub : 0.f;
-                            wsum = fa(wsum, w);
-                            ax = fa(ax, fm(xi.x, w));
-                            ay = fa(ay, fm(xi.y, w));
-                            az = fa(az, fm(xi.z, w));
-                        }
-                    } else {
-                        // SphSDF: (mass / rho) W_std(d) at radius R (kernel.cpp:123-132)
-                        const float d2 = fm(d, d);
-                        const float of = fs(d2, A.r2);
-                        float w = 0.f;
-                        if (!(fabsf(of) < A.iz || of > 0.f)) {
-                            w = double_cube(A.wc, A.wh, A.wl, fs(1.f, fdv(d2, A.r2)));
-                        }
-                        wsum = fa(wsum, fm(fdv(A.mass, A.rho[s]), w));
-                    }
-                }
+    auto add = [&](unsigned s, float4 xi) {
+        const float d = dist3(p, xi);
+        if (A.method == 0) {
+            // ZhuBridsonSDF: k_cub(|p - x| / R) = Max(0, (1 - s^2)^3), the cube in double
+            if (d < R) {
+                const float t = fdv(d, R);
+                const float cub = double_cube_1m(fm(t, t));
+                const float w = 0.f < cub ? cub : 0.f;
+                wsum = fa(wsum, w);
+                ax = fa(ax, fm(xi.x, w));
+                ay = fa(ay, fm(xi.y, w));
+                az = fa(az, fm(xi.z, w));
             }
+        } else {
+            // SphSDF: (mass / rho) W_std(d) at radius R (kernel.cpp:123-132)
+            const float d2 = fm(d, d);
+            const float of = fs(d2, A.r2);
+            float w = 0.f;
+            if (!(fabsf(of) < A.iz || of > 0.f)) {
+                w = double_cube(A.wc, A.wh, A.wl, fs(1.f, fdv(d2, A.r2)));
+            }
+            wsum = fa(wsum, fm(fdv(A.mass, A.rho[s]), w));
+        }
+    };
+    int kept = 0;
+    auto flush = [&]() {
+        for (int q = 0; q < kept; q += 4) {
+            unsigned s[4];
+            float4 x[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) s[u] = near[min(q + u, kept - 1)][t];
+#pragma unroll
+            for (int u = 0; u < 4; u++) x[u] = __ldg(&A.pos[s[u]]);
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (q + u < kept) add(s[u], x[u]);
+        }
+        kept = 0;
+    };
+    const unsigned plane = (unsigned)g.nx * (unsigned)g.ny;
+    const unsigned z0 = (unsigned)max(cz - 1, 0), z1 = (unsigned)min(cz + 1, g.nz - 1);
+    for (int y = max(cy - 1, 0); y <= min(cy + 1, g.ny - 1); y++)
+        for (int x = max(cx - 1, 0); x <= min(cx + 1, g.nx - 1); x++) {
+            const unsigned row = (unsigned)x + (unsigned)y * g.nx;
+            unsigned b[3], e[3];
+#pragma unroll
+            for (int z = 0; z < 3; z++) {
+                const unsigned nb = row + min(z0 + z, z1) * plane;
+                b[z] = __ldg(&A.start[nb]);
+                e[z] = z0 + z <= z1 ? __ldg(&A.start[nb + 1]) : b[z];
+            }
+#pragma unroll
+            for (int z = 0; z < 3; z++)
+                for (unsigned s = b[z]; s < e[z]; s += 4) {
+                    float4 xi[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) xi[u] = __ldg(&A.pos[min(s + u, e[z] - 1u)]);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const float ex = fs(p.x, xi[u].x), ey = fs(p.y, xi[u].y), ez = fs(p.z, xi[u].z);
+                        const float d2 = fa(fa(fm(ex, ex), fm(ey, ey)), fm(ez, ez));
+                        near[kept][t] = s + u;
+                        kept += s + u < e[z] && (A.method != 0 || d2 <= A.near2) ? 1 : 0;
+                    }
+                    if (kept > kFieldSlots - 5) flush();
+                }
+        }
+    flush();
     if (A.method != 0) {
         out[i] = fs(0.5f, wsum);
     } else if (wsum > 0.f) {
@@ -85,7 +134,7 @@ __global__ void k_particle_sdf(SurfaceArgs A, float *__restrict__ out) {
 
 void launch_particle_sdf(const SurfaceArgs &A, float *out, cudaStream_t s) {
     const long long total = (long long)A.nodes[0] * A.nodes[1] * A.nodes[2];
-    k_particle_sdf<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(A, out);
+    k_particle_sdf<<<(unsigned)((total + kFieldThreads - 1) / kFieldThreads), kFieldThreads, 0, s>>>(A, out);
 }
 
 }  // namespace bbg
