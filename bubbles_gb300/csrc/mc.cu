@@ -128,33 +128,46 @@ __device__ __forceinline__ int cube_config(const McGrid &g, int i, int j, int k)
 }
 
 // cube index with x slowest and z fastest, the reference's cubeId order
-__device__ __forceinline__ void cube_of(const McGrid &g, long long id, int &i, int &j, int &k) {
-    const long long zl = g.nz - 1, yl = g.ny - 1;
-    k = (int)(id % zl);
-    j = (int)((id / zl) % yl);
-    i = (int)(id / (yl * zl));
+// (three entries a node fit 31 bits, so 32-bit divisions do)
+__device__ __forceinline__ void cube_of(const McGrid &g, unsigned id, int &i, int &j, int &k) {
+    const unsigned zl = (unsigned)g.nz - 1u, yl = (unsigned)g.ny - 1u;
+    const unsigned row = id / zl;
+    k = (int)(id - row * zl);
+    i = (int)(row / yl);
+    j = (int)(row - (unsigned)i * yl);
+}
+
+__device__ __forceinline__ void node_of(const McGrid &g, unsigned n, int &i, int &j, int &k) {
+    const unsigned row = n / (unsigned)g.nx;
+    i = (int)(n - row * (unsigned)g.nx);
+    k = (int)(row / (unsigned)g.ny);
+    j = (int)(row - (unsigned)k * (unsigned)g.ny);
 }
 
 __global__ void k_mc_cubes(McGrid g, long long cubes, unsigned *__restrict__ ntri) {
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= cubes) return;
     int i, j, k;
-    cube_of(g, id, i, j, k);
+    cube_of(g, (unsigned)id, i, j, k);
     ntri[id] = (unsigned)case_triangles(cube_config(g, i, j, k));
 }
 
-// edge e = axis * nodes + node: the edge from node (i, j, k) along the axis
-__global__ void k_mc_edges(McGrid g, long long nodes, unsigned *__restrict__ crossing) {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= 3 * nodes) return;
-    const int axis = (int)(e / nodes);
-    const long long n = e - axis * nodes;
-    const int i = (int)(n % g.nx), j = (int)((n / g.nx) % g.ny), k = (int)(n / ((long long)g.nx * g.ny));
-    const int i1 = i + (axis == 0), j1 = j + (axis == 1), k1 = k + (axis == 2);
-    unsigned c = 0;
-    if (i1 < g.nx && j1 < g.ny && k1 < g.nz)
-        c = ((node_value(g, i, j, k) <= g.iso) != (node_value(g, i1, j1, k1) <= g.iso)) ? 1u : 0u;
-    crossing[e] = c;
+// edge e = axis * nodes + node: the edge from node (i, j, k) along the axis.  A thread per node writes its
+// three edges, and both copies of the flags: the scan consumes one.
+__global__ void k_mc_edges(McGrid g, long long nodes, unsigned *__restrict__ crossing, unsigned *__restrict__ copy) {
+    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= nodes) return;
+    int i, j, k;
+    node_of(g, (unsigned)n, i, j, k);
+    const bool in = node_value(g, i, j, k) <= g.iso;
+#pragma unroll
+    for (int axis = 0; axis < 3; axis++) {
+        const int i1 = i + (axis == 0), j1 = j + (axis == 1), k1 = k + (axis == 2);
+        unsigned c = 0;
+        if (i1 < g.nx && j1 < g.ny && k1 < g.nz) c = in != (node_value(g, i1, j1, k1) <= g.iso) ? 1u : 0u;
+        crossing[axis * nodes + n] = c;
+        copy[axis * nodes + n] = c;
+    }
 }
 
 // grad (marching_cubes.cpp:121-159): central differences, one-sided at the first node and
@@ -184,9 +197,9 @@ __global__ void k_mc_vertices(McGrid g, long long nodes, const unsigned *__restr
                               float *__restrict__ normals) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= 3 * nodes || !crossing[e]) return;
-    const int axis = (int)(e / nodes);
-    const long long n = e - axis * nodes;
-    const int i = (int)(n % g.nx), j = (int)((n / g.nx) % g.ny), k = (int)(n / ((long long)g.nx * g.ny));
+    const int axis = e >= 2 * nodes ? 2 : e >= nodes ? 1 : 0;
+    int i, j, k;
+    node_of(g, (unsigned)(e - axis * nodes), i, j, k);
     const int i1 = i + (axis == 0), j1 = j + (axis == 1), k1 = k + (axis == 2);
     // distanceToZeroLevelSet, clamped to [1e-6, 0.999999]
     const float phi0 = fs(node_value(g, i, j, k), g.iso), phi1 = fs(node_value(g, i1, j1, k1), g.iso);
@@ -213,7 +226,7 @@ __global__ void k_mc_triangles(McGrid g, long long cubes, long long nodes, const
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= cubes) return;
     int i, j, k;
-    cube_of(g, id, i, j, k);
+    cube_of(g, (unsigned)id, i, j, k);
     const int cfg = cube_config(g, i, j, k);
     const int nt = case_triangles(cfg);
     unsigned t0 = tri_start[id];
@@ -266,9 +279,7 @@ cudaError_t mc_count(const McInput &in, unsigned *ntri_cube, unsigned *tri_start
     const long long nodes = (long long)g.nx * g.ny * g.nz;
     k_mc_cubes<<<blocks_for(cubes, 256), 256, 0, s>>>(g, cubes, ntri_cube);
     launch_cell_scan(ntri_cube, (unsigned)cubes, tri_part, tri_start, s);
-    k_mc_edges<<<blocks_for(3 * nodes, 256), 256, 0, s>>>(g, nodes, crossing);
-    // the scan zeroes its input: keep the crossing flags, scan a copy
-    cudaMemcpyAsync(flag_copy, crossing, sizeof(unsigned) * (size_t)(3 * nodes), cudaMemcpyDeviceToDevice, s);
+    k_mc_edges<<<blocks_for(nodes, 256), 256, 0, s>>>(g, nodes, crossing, flag_copy);
     launch_cell_scan(flag_copy, (unsigned)(3 * nodes), v_part, vindex, s);
     cudaMemcpyAsync(h, tri_start + cubes, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(h + 1, vindex + 3 * nodes, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
