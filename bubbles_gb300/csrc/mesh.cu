@@ -262,7 +262,10 @@ constexpr int kMaxRayHits = 256;   // a ray stuck on degenerate geometry gives u
 //    growth, the test of the reference's BVH) rejects the box for the current tMax, which
 //    never rejects a box holding a hit at or before tMax.
 constexpr int kMeshTile = 64;
-constexpr int kMeshSub = 8;
+// Sub-tiles of 4 leave fewer triangles for twice the box tests inside a kept tile: the torus below, the whole
+// call, 1,270 -> 1,091 us against 8 (of 2: 1,126; tiles of 32 with 4: 1,100, and twice the tiles to pass
+// over in a large mesh).
+constexpr int kMeshSub = 4;
 
 // Boxes: 8 floats each, low corner then high corner.  Squared distance of p to a box:
 __device__ __forceinline__ float box_distance2(const float4 *__restrict__ bx, v3 p) {
@@ -297,7 +300,8 @@ __device__ __forceinline__ void mesh_walk(const float4 *__restrict__ tiles, int 
 // Bound: FP32 issue slots of the triangle tests that the boxes leave.  The lanes of a warp share
 // them when their nodes are near one another in all three directions: 22.7 of 32 lanes active a
 // triangle with bricks, 12.9 with 32 nodes in a row.  Torus of 1,152 triangles, 0.43M nodes: 23.0
-// ms with the double products per node, 1.49 ms without, 0.88 ms in bricks.
+// ms with the double products per node, 1.49 ms without, 0.88 ms in bricks, 0.74 ms with sub-tiles of
+// 4 (rays 0.35 of it before).
 __global__ void __launch_bounds__(128)
 k_mesh_sdf(const float4 *__restrict__ ray, int ntri, const float4 *__restrict__ tiles, const float4 *__restrict__ dist,
            const float4 *__restrict__ dtiles, float margin, SdfDev g, v3 lo, v3 hi, Gammas G, float *__restrict__ out,
