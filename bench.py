@@ -56,8 +56,8 @@ def alg_bytes(list_len):
     return {
         "k_hash_count": 16 + 4 + 4,                        # pos in; cell, arrival index out
         "k_place": 4 + 4 + 4 + 4 + 8,                      # cell, index, start, id in; (id, slot) out
-        "k_rank_gather": 8 + 4 + 4 + 32 + 32 + 4 + 4 + 4 + 4 + 4,  # + pressure in, previous pressure out
-        "k_density": 16 + 4 + 4 + 4 + 4 + 4 + L,          # pos, cell in; rho, 1/rho, vel.w, count, list out
+        "k_rank_gather": 8 + 4 + 4 + 32 + 32 + 4 + 4 + 4 + 4 + 4 + 8,  # + pressure in, previous pressure, filter record out
+        "k_density": 16 + 8 + 4 + 4 + 4 + 4 + 4 + L,      # pos, filter record, cell in; rho, 1/rho, vel.w, count, list out
         "k_non_pressure": 16 + 16 + 4 + 4 + 16 + 4 + 16 + 16 + L,  # pos, vel, cell, count, list; F, p, Fp, x* out
         "k_pred_density": 16 + 4 + 4 + 4 + 4 + 4 + 4 + 4 + L,     # x*, cell, count, list, p; p, rho*, err, pos.w
         "k_pressure_force": 16 + 16 + 4 + 4 + 16 + 16 + 16 + L,   # pos, vel, cell, count, list, F; Fp, x* out
@@ -308,15 +308,14 @@ def cpu_sample(scene, pos, vel, depth):
 
 def launches_per_substep(scene, variant, iters, worklist=1):
     """Kernels one graph-launched PCISPH substep runs: 5 for the grid rebuild (hash and
-    count, 2 scan kernels, place, rank and gather), 2 for density (the pair-record copy and
-    the pass), non-pressure, 3 per corrector iteration (predicted density, pressure force,
-    loop control), plus the warm start (one kernel; learned: features and the MLP); 2 more
+    count, 2 scan kernels, place, rank and gather), density, non-pressure, 2 per corrector
+    iteration (predicted density, pressure force), plus the warm start (one kernel; learned: features and the MLP); 2 more
     when pseudo-viscosity is active.  A batch adds the scenes' slot ranges and, with a work
     list, its rebuild before each iteration."""
     pv = 2 if scene.get("pseudo_viscosity", 10.0) * scene["dt"] > 0.1 else 0
     extra = {"plain": 0, "warm": 1, "learned": 2}[variant]
     batch = (1 + (iters if worklist else 0)) if scene.get("batch") else 0
-    return 8 + extra + 3 * iters + pv + batch
+    return 7 + extra + 2 * iters + pv + batch
 
 
 def sample_substeps(first, total, k):
@@ -467,7 +466,7 @@ def seeding(bb, scene, final_pos, device, reps=3):
     s2.close()
     out["mesh_sdf"] = {"triangles": len(tris), "nodes": int(np.prod(nodes)), "ms": 1e3 * min(t),
                        "inside_nodes": int((vals < 0).sum()), "stuck_rays": stuck,
-                       "note": "tiles of 64 and sub-tiles of 8 triangles culled by their boxes (distance over a Morton-ordered copy, rays in index order)"}
+                       "note": "tiles of 64 and sub-tiles of 4 triangles culled by their boxes (distance over a Morton-ordered copy, rays in index order)"}
     out["measured"] = "host wall clock around the C-ABI calls (single call; emitter median of %d)" % reps
     return out
 

@@ -15,9 +15,10 @@
 // mma.sync m16n8k16 (a warp evaluates 16 particles per pass: 8 MMAs for layer 1 with
 // the bias folded in as a constant input, 32 for layer 2; layer 3 is a 64-term dot
 // product on the FP32 pipes reduced across the quad).  Training is FP32 on the CUDA
-// cores: one block of 128 samples per CTA computes the forward pass, back-propagates
-// the squared error and reduces its weight gradients in shared memory; an Adam kernel
-// updates the FP32 master parameters and rebuilds the BF16 fragments.
+// cores: a block takes 128 samples at a time through the forward pass, back-propagates
+// the squared error and sums its weight gradients into a row of its own; an Adam kernel
+// adds the rows and updates the FP32 master parameters, and a third rebuilds the BF16
+// fragments.
 #include "bbg_kernels.h"
 #include "mlp.h"
 
