@@ -236,13 +236,13 @@ constexpr int kMasks = 10;
 // particle's neighbour set (the reference bucket, grid.h:423-447) as a member list.  A thread per
 // particle, in two phases.
 //
-// Filter: all candidates of the 27 cells (about 216), eight at a time from k_filter_records' halves:
+// Filter: all candidates of the 27 cells (about 216), eight at a time from the halves the grid update's gather wrote:
 // the sign of P.filt - r^2, the squared radius widened by the rounding of the halves, into a
 // mask of 32 aligned slots, and nothing else.  It only leaves out what cannot be a member.
 // Members: the exact test, the kernel sum in float and the list over the about 29 candidates left.
 //
-// Measured at 1,048,576 particles (with the records' launch): 234 -> 156 us; 4,194,304: 866 -> 578;
-// 262,144: 78 -> 52.  The pass that tested and summed every candidate in float was bound by issue
+// Measured at 1,048,576 particles: 234 -> 149 us; 4,194,304: 866 -> 554; 262,144: 78 -> 47 (with a
+// records' launch of its own: 156, 578, 52).  The pass that tested and summed every candidate in float was bound by issue
 // slots (256 M warp instructions, 83 %); this one issues 136 M.  The filter's bound is the FMA
 // pipe (24 half2 operations per eight candidates); with float candidates it was L1, whose 128 bytes
 // a clock return 12 bytes a candidate to every lane (181 us), half of that as halves.  A warp per
