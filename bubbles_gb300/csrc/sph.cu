@@ -132,6 +132,12 @@ struct DensitySum {
         listed += other ? 1 : 0;
         self += mem && !other ? 1 : 0;
     }
+    // past the work cap: the particle itself only
+    __device__ __forceinline__ void crowded(StepState *st) {
+        atomicAdd(&st->crowded, 1u);
+        sum = 1.f;
+        self = 1;
+    }
 };
 
 // The end of the density pass for particle i: density, equation of state, counters.
@@ -156,15 +162,13 @@ __device__ __forceinline__ void density_store(const Params &P, float4 *pos, floa
     if (cnt > kBucketCap) atomicAdd(&st->nbr_overflow, 1u);
 }
 
-// Candidates one by one (a particle whose candidates do not fit the filter's masks), counted
-// as crowded past the work cap: the particle itself only.
+// Candidates one by one (a particle with more members than its lanes keep), counted as crowded past
+// the work cap.
 __device__ __forceinline__ void density_walk(const Params &P, const float4 *__restrict__ pos,
                                              const unsigned *__restrict__ start, unsigned c, float4 pi, unsigned i,
                                              StepState *st, DensitySum &D) {
     if (candidate_count(P.g, start, c) > kMaxCandidates) {
-        atomicAdd(&st->crowded, 1u);
-        D.sum = 1.f;
-        D.self = 1;
+        D.crowded(st);
         return;
     }
     tile_rows(P.g, start, c, [&](int, unsigned b, unsigned e) {
@@ -229,8 +233,117 @@ __device__ __forceinline__ unsigned half2_bits(__half2 v) { return *reinterpret_
 __device__ __forceinline__ __half2 as_half2(unsigned v) { return *reinterpret_cast<__half2 *>(&v); }
 
 // Masks a particle keeps between the filter and the member phase of k_density_mask: 9 rows and
-// one more for a row whose slots span more than 32.
+// one more for a row whose slots span more than 32.  Denser particles (the rest density compressed by a
+// third, or a wider kernel) take the two phases in several rounds: 1,000,000 particles at 1.63 times the rest
+// density 265 us (walked one candidate after another they took 628), at 1.17 times, one round, 158.
+// The further rounds are compiled to fit the first one's 56 registers, 9 blocks an SM: with 61 to 64 of them
+// the single-round states took 3 % longer.
 constexpr int kMasks = 10;
+
+// The filter of k_density_mask for the particle at pi in cell c: the non-empty masks of its
+// candidates, entry k at keep[k * stride].  Returns their number, or when kMasks have no room for
+// them ~s, s the slot to go on from: with RESUME, from there, one mask fewer at a time.
+// total: the candidates of the 27 cells.
+template <bool FEW, bool RESUME>
+__device__ __forceinline__ int density_filter(const Params &P, const unsigned *__restrict__ start,
+                                              const uint4 *__restrict__ rec, float4 pi, unsigned c, uint2 *keep,
+                                              int stride, unsigned from, unsigned &total) {
+    constexpr int room = RESUME ? kMasks - 1 : kMasks;
+    int kept = 0;
+    total = 0;
+    const GridDev &g = P.g;
+    int cx, cy, cz;
+    cell_coords(g, c, cx, cy, cz);
+    const v3 f = filter_offset(P, pi, cx, cy, cz);
+    const int far = ((cx + 1) & 2) ? 0 : 1;   // cells 1 and 2 of the first window, else the second
+    const __half2 X = __float2half2_rn((float)(((cx + 2 * far) & 3) - 2) * P.filt_side[0] + f.x);
+    const __half2 T = as_half2(P.filt);
+    // rows x, y, z of a record, or y, z, x' of the second window: the test takes the axes in any order
+    const uint4 *const rec0 = rec + far;
+    const int x0 = cx > 0 ? -1 : 0, x1 = cx + 1 < g.nx ? 2 : 1;
+    const int plane = g.nx * g.ny;
+    // row r = 3 (dz + 1) + dy + 1, inside the grid or empty; the next row's range is requested a row
+    // ahead (with RESUME not, for its registers)
+    unsigned inside = 0x1ffu;
+    if (cy == 0) inside &= ~0x049u;
+    if (cy + 1 >= g.ny) inside &= ~0x124u;
+    if (cz == 0) inside &= ~0x007u;
+    if (cz + 1 >= g.nz) inside &= ~0x1c0u;
+    int row = (int)c - g.nx - plane;
+    unsigned nb = 0, ne = 0;
+    auto range = [&]() {
+        nb = ne = 0;
+        if (inside & 1u) {
+            nb = __ldg(&start[row + x0]);
+            ne = __ldg(&start[row + x1]);
+        }
+    };
+    if (!RESUME) range();
+    __half2 Z = __float2half2_rn(f.z + 0.5f * P.filt_side[2]);
+    float fy = f.y + 0.5f * P.filt_side[1];
+    int dy = 0;
+#pragma unroll 1
+    for (int r = 0; r < 9; r++) {
+        if (RESUME) range();
+        const unsigned b = nb, e = ne;
+        const __half2 Y = __float2half2_rn(fy);
+        const __half2 A = far ? Y : X, B = far ? Z : Y, C = far ? X : Z;
+        fy -= P.filt_side[1];
+        row += g.nx;
+        if (++dy == 3) {
+            dy = 0;
+            row += plane - 3 * g.nx;
+            fy = f.y + 0.5f * P.filt_side[1];
+            Z = __float2half2_rn(f.z + (r == 2 ? -0.5f : -1.5f) * P.filt_side[2]);
+        }
+        inside >>= 1;
+        if (!RESUME) range();
+        total += e - b;
+        for (unsigned cb = RESUME && from > b ? from : b & ~7u; cb < e; cb += 32u) {
+            const unsigned span = min(32u, e - cb);
+            const int groups = (int)((span + 7u) >> 3);
+            const uint4 *q = rec0 + (size_t)(cb >> 3) * 4u;
+            unsigned m = 0;
+            auto group = [&](const uint4 &a, const uint4 &v, const uint4 &w) {
+                auto test = [&](unsigned ua, unsigned ub, unsigned uc) {
+                    const __half2 da = __hsub2(as_half2(ua), A), db = __hsub2(as_half2(ub), B);
+                    const __half2 dc = __hsub2(as_half2(uc), C);
+                    return half2_bits(__hfma2(__hneg2(da), da, __hfma2(__hneg2(db), db, __hfma2(__hneg2(dc), dc, T))));
+                };
+                const unsigned w0 = test(a.x, v.x, w.x), w1 = test(a.y, v.y, w.y);
+                const unsigned w2 = test(a.z, v.z, w.z), w3 = test(a.w, v.w, w.w);
+                // the eight signs (set: outside) as a byte, the first slot its top bit
+                unsigned s = __dp4a(__byte_perm(w0, w1, 0x7531) & 0x80808080u, 0x10204080u, 0u);
+                s = __dp4a(__byte_perm(w2, w3, 0x7531) & 0x80808080u, 0x01020408u, s);
+                m = (m << 8) + (s >> 7);
+            };
+            if (FEW) {
+                uint4 a[4], v[4], w[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const uint4 *g4 = q + 4 * min(k, groups - 1);
+                    a[k] = __ldg(g4);
+                    v[k] = __ldg(g4 + 1);
+                    w[k] = __ldg(g4 + 2);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (k < groups) group(a[k], v[k], w[k]);
+            } else {
+                for (int k = 0; k < groups; k++, q += 4) group(__ldg(q), __ldg(q + 1), __ldg(q + 2));
+            }
+            m = ~m << (32 - 8 * groups);
+            // the slots of [b, e) only
+            if (b > cb) m &= 0xffffffffu >> (b - cb);
+            m &= (unsigned)((int)0x80000000 >> (span - 1u));
+            if (m) {
+                if ((unsigned)kept < (unsigned)room) keep[kept++ * stride] = make_uint2(m, cb);
+                else if (kept == room) kept = ~(int)max(cb, b);
+            }
+        }
+    }
+    return kept;
+}
 
 // The density pass: ComputeDensityFor + ComputePressureValue (sph_equations3.cpp:7-58), and each
 // particle's neighbour set (the reference bucket, grid.h:423-447) as a member list.  A thread per
@@ -264,102 +377,24 @@ k_density_mask(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, uns
     const int stride = (int)blockDim.x;
     const float4 pi = pos[i];
     const unsigned cw = cell[i], c = cw & ~kWide;
-    int kept = 0;
-    unsigned total = 0;
-    {
-        const GridDev &g = P.g;
-        int cx, cy, cz;
-        cell_coords(g, c, cx, cy, cz);
-        const v3 f = filter_offset(P, pi, cx, cy, cz);
-        const int far = ((cx + 1) & 2) ? 0 : 1;   // cells 1 and 2 of the first window, else the second
-        const __half2 X = __float2half2_rn((float)(((cx + 2 * far) & 3) - 2) * P.filt_side[0] + f.x);
-        const __half2 T = as_half2(P.filt);
-        // rows x, y, z of a record, or y, z, x' of the second window: the test takes the axes in any order
-        const uint4 *const rec0 = rec + far;
-        const int x0 = cx > 0 ? -1 : 0, x1 = cx + 1 < g.nx ? 2 : 1;
-        const int plane = g.nx * g.ny;
-        // row r = 3 (dz + 1) + dy + 1, inside the grid or empty; the next row's range is requested a row ahead
-        unsigned inside = 0x1ffu;
-        if (cy == 0) inside &= ~0x049u;
-        if (cy + 1 >= g.ny) inside &= ~0x124u;
-        if (cz == 0) inside &= ~0x007u;
-        if (cz + 1 >= g.nz) inside &= ~0x1c0u;
-        int row = (int)c - g.nx - plane;
-        unsigned nb = 0, ne = 0;
-        if (inside & 1u) {
-            nb = __ldg(&start[row + x0]);
-            ne = __ldg(&start[row + x1]);
-        }
-        __half2 Z = __float2half2_rn(f.z + 0.5f * P.filt_side[2]);
-        float fy = f.y + 0.5f * P.filt_side[1];
-        int dy = 0;
-#pragma unroll 1
-        for (int r = 0; r < 9; r++) {
-            const unsigned b = nb, e = ne;
-            const __half2 Y = __float2half2_rn(fy);
-            const __half2 A = far ? Y : X, B = far ? Z : Y, C = far ? X : Z;
-            fy -= P.filt_side[1];
-            row += g.nx;
-            if (++dy == 3) {
-                dy = 0;
-                row += plane - 3 * g.nx;
-                fy = f.y + 0.5f * P.filt_side[1];
-                Z = __float2half2_rn(f.z + (r == 2 ? -0.5f : -1.5f) * P.filt_side[2]);
-            }
-            inside >>= 1;
-            nb = ne = 0;
-            if (inside & 1u) {
-                nb = __ldg(&start[row + x0]);
-                ne = __ldg(&start[row + x1]);
-            }
-            total += e - b;
-            for (unsigned cb = b & ~7u; cb < e; cb += 32u) {
-                const unsigned span = min(32u, e - cb);
-                const int groups = (int)((span + 7u) >> 3);
-                const uint4 *q = rec0 + (size_t)(cb >> 3) * 4u;
-                unsigned m = 0;
-                auto group = [&](const uint4 &a, const uint4 &v, const uint4 &w) {
-                    auto test = [&](unsigned ua, unsigned ub, unsigned uc) {
-                        const __half2 da = __hsub2(as_half2(ua), A), db = __hsub2(as_half2(ub), B);
-                        const __half2 dc = __hsub2(as_half2(uc), C);
-                        return half2_bits(__hfma2(__hneg2(da), da, __hfma2(__hneg2(db), db, __hfma2(__hneg2(dc), dc, T))));
-                    };
-                    const unsigned w0 = test(a.x, v.x, w.x), w1 = test(a.y, v.y, w.y);
-                    const unsigned w2 = test(a.z, v.z, w.z), w3 = test(a.w, v.w, w.w);
-                    // the eight signs (set: outside) as a byte, the first slot its top bit
-                    unsigned s = __dp4a(__byte_perm(w0, w1, 0x7531) & 0x80808080u, 0x10204080u, 0u);
-                    s = __dp4a(__byte_perm(w2, w3, 0x7531) & 0x80808080u, 0x01020408u, s);
-                    m = (m << 8) + (s >> 7);
-                };
-                if (FEW) {
-                    uint4 a[4], v[4], w[4];
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const uint4 *g4 = q + 4 * min(k, groups - 1);
-                        a[k] = __ldg(g4);
-                        v[k] = __ldg(g4 + 1);
-                        w[k] = __ldg(g4 + 2);
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        if (k < groups) group(a[k], v[k], w[k]);
-                } else {
-                    for (int k = 0; k < groups; k++, q += 4) group(__ldg(q), __ldg(q + 1), __ldg(q + 2));
-                }
-                m = ~m << (32 - 8 * groups);
-                // the slots of [b, e) only
-                if (b > cb) m &= 0xffffffffu >> (b - cb);
-                m &= (unsigned)((int)0x80000000 >> (span - 1u));
-                if (m) {
-                    if (kept < kMasks) keep[kept * stride] = make_uint2(m, cb);
-                    kept++;
-                }
-            }
+    unsigned total;
+    int kept = density_filter<FEW, false>(P, start, rec, pi, c, keep, stride, 0u, total);
+    DensitySum D(list + i);
+    if (total > kMaxCandidates) {
+        D.crowded(st);
+    } else {
+        density_members<FEW ? 8 : 4>(P, pos, pi, (unsigned)i, D, keep, stride, kept < 0 ? kMasks : kept);
+        while (kept < 0) {   // the rest; the last entry keeps the sums meanwhile
+            keep[(kMasks - 1) * stride] = make_uint2(__float_as_uint(D.sum), 2u * (unsigned)D.listed + (unsigned)D.self);
+            kept = density_filter<FEW, true>(P, start, rec, pi, c, keep, stride, ~(unsigned)kept, total);
+            const uint2 d = keep[(kMasks - 1) * stride];
+            D.sum = __uint_as_float(d.x);
+            D.listed = (int)(d.y >> 1);
+            D.self = (int)(d.y & 1u);
+            D.out = list + i + (size_t)D.listed * P.n;
+            density_members<FEW ? 8 : 4>(P, pos, pi, (unsigned)i, D, keep, stride, kept < 0 ? kMasks - 1 : kept);
         }
     }
-    DensitySum D(list + i);
-    if (kept > kMasks || total > kMaxCandidates) density_walk(P, pos, start, c, pi, (unsigned)i, st, D);
-    else density_members<FEW ? 8 : 4>(P, pos, pi, (unsigned)i, D, keep, stride, kept);
     density_store(P, pos, vel, cell, rho, inv_rho, press, nbr, compute_pressure, st, i, pi, cw, D.sum,
                   D.listed + D.self, D.listed);
 }
