@@ -132,12 +132,6 @@ struct DensitySum {
         listed += other ? 1 : 0;
         self += mem && !other ? 1 : 0;
     }
-    // past the work cap: the particle itself only
-    __device__ __forceinline__ void crowded(StepState *st) {
-        atomicAdd(&st->crowded, 1u);
-        sum = 1.f;
-        self = 1;
-    }
 };
 
 // The end of the density pass for particle i: density, equation of state, counters.
@@ -160,24 +154,6 @@ __device__ __forceinline__ void density_store(const Params &P, float4 *pos, floa
     if (P.nscenes > 0) P.scene[i] = (unsigned short)scene_of(P, pi.z);
     if (listed > kMaxList) cell[i] = cw | kWide;
     if (cnt > kBucketCap) atomicAdd(&st->nbr_overflow, 1u);
-}
-
-// Candidates one by one (a particle with more members than its lanes keep), counted as crowded past
-// the work cap.
-__device__ __forceinline__ void density_walk(const Params &P, const float4 *__restrict__ pos,
-                                             const unsigned *__restrict__ start, unsigned c, float4 pi, unsigned i,
-                                             StepState *st, DensitySum &D) {
-    if (candidate_count(P.g, start, c) > kMaxCandidates) {
-        D.crowded(st);
-        return;
-    }
-    tile_rows(P.g, start, c, [&](int, unsigned b, unsigned e) {
-        for (unsigned j = b; j < e; ++j) {
-            const float4 pj = __ldg(&pos[j]);
-            const float r2 = DensitySum::dist(pi, pj);
-            D.take(P, std_member(P, pi, pj, r2), r2, j, i);
-        }
-    });
 }
 
 // The member phase over `kept` non-empty masks of candidates, entry k at keep[k * stride]: (mask,
@@ -381,7 +357,9 @@ k_density_mask(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, uns
     int kept = density_filter<FEW, false>(P, start, rec, pi, c, keep, stride, 0u, total);
     DensitySum D(list + i);
     if (total > kMaxCandidates) {
-        D.crowded(st);
+        atomicAdd(&st->crowded, 1u);   // the particle itself only
+        D.sum = 1.f;
+        D.self = 1;
     } else {
         density_members<FEW ? 8 : 4>(P, pos, pi, (unsigned)i, D, keep, stride, kept < 0 ? kMasks : kept);
         while (kept < 0) {   // the rest; the last entry keeps the sums meanwhile
@@ -407,7 +385,7 @@ k_density_mask(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, uns
 // SPH substeps, 8 and 4 lanes 340, a thread each 371; 16,384: 8 and 4 lanes 370, a thread each 375; 20,000:
 // no difference; 35,937, 4 lanes: 461 against 374).
 constexpr int kGroupThreads = 128;
-constexpr int kGroupMembers = kMaxList;   // a particle with more (itself counted) is walked by one lane
+constexpr int kGroupMembers = kMaxList;   // of a particle (itself counted) in shared memory at a time
 constexpr int kGroup16 = 152 * 8 * kGroupThreads / 16;   // particles, up to
 constexpr int kGroup8 = 2 * kGroup16;
 
@@ -429,7 +407,7 @@ k_density_group(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, un
     __shared__ unsigned row_off[9][S];   // slot of a candidate of the row less its number
     __shared__ float term[kGroupMembers][S];
     __shared__ ListEntry member[kGroupMembers][S];
-    __shared__ int found[S], itself[S];   // members (-1: walked); the particle itself one
+    __shared__ int found[S], itself[S];   // members (-1: past the work cap); the particle itself one
     constexpr unsigned full = 0xffffffffu, group = (1u << G) - 1u;
     const int grp = threadIdx.x / G, lane = threadIdx.x & (G - 1);
     const int shift = threadIdx.x & 31 & ~(G - 1);
@@ -502,36 +480,73 @@ k_density_group(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, un
             if (mem[u] && q < kGroupMembers) {
                 const float x = __fmaf_rn(-r2, P.inv_h2, 1.f);
                 term[q][grp] = __fmul_rn(__fmul_rn(x, x), x);
-                // the list leaves the particle itself out
+                // the list leaves the particle itself out (and its last entry, if members are left, to come)
                 if (j[u] != (unsigned)i) member[q - (j[u] > (unsigned)i ? self : 0)][grp] = j[u];
             }
         }
     }
     if (lane == 0) {
-        found[grp] = !live ? 0 : total > kMaxCandidates || cnt > kGroupMembers ? -1 : cnt;
+        found[grp] = !live ? 0 : total > kMaxCandidates ? -1 : cnt;
         itself[grp] = self;
     }
-    __syncthreads();
+    const bool more = __syncthreads_or(cnt > kGroupMembers);
     const int mine = threadIdx.x & (S - 1);
-    cnt = found[mine];
-    const int listed = cnt - itself[mine];
+    const int all = found[mine], listed = all - itself[mine];
+    float sum = 0.f;
     if (threadIdx.x >= 32) {   // the lists, rows of the block's particles together
-        for (int q = (threadIdx.x - 32) / S; q < listed; q += (kGroupThreads - 32) / S)
+        for (int q = (threadIdx.x - 32) / S; q < min(listed, kMaxList); q += (kGroupThreads - 32) / S)
             list[(size_t)q * P.n + i0 + mine] = member[q][mine];
-    } else if (threadIdx.x < S && i0 + mine < P.n) {
+    } else if (threadIdx.x < S) {
+        const int some = min(all, kGroupMembers);
+#pragma unroll 8
+        for (int q = 0; q < some; q++) sum = __fadd_rn(sum, term[q][mine]);
+    }
+    // The block's particles with more members than that (a dense state, a wider kernel): the candidates
+    // again for the next ones.  15,625 particles of 93 members: 151 us when a lane of each walked them
+    // alone, 54 now; none of a state of 28 members pays for it (14.4 us).
+    if (more) {
+        for (int base = kGroupMembers;; base += kGroupMembers) {
+            __syncthreads();   // the terms are added, the lists written
+            cnt = r = 0;
+            rend = row_end[0][grp];
+            roff = row_off[0][grp];
+#pragma unroll 4
+            for (unsigned k = lane; k < longest + lane; k += G) {
+                bool mem = k < work;
+                while (mem && k >= rend) {
+                    r++;
+                    rend = row_end[r][grp];
+                    roff = row_off[r][grp];
+                }
+                const unsigned j = mem ? roff + k : (unsigned)i;
+                const float4 pj = __ldg(&pos[j]);
+                const float r2 = DensitySum::dist(pi, pj);
+                mem = mem && std_member(P, pi, pj, r2);
+                const unsigned m = (__ballot_sync(full, mem) >> shift) & group;
+                const int q = cnt + __popc(m & ((1u << lane) - 1u)) - base;
+                cnt += __popc(m);
+                if (mem && q >= 0 && q < kGroupMembers) {
+                    const float x = __fmaf_rn(-r2, P.inv_h2, 1.f);
+                    term[q][grp] = __fmul_rn(__fmul_rn(x, x), x);
+                    // the last entry of the list, where the particle itself came before
+                    if (base + q == kMaxList && self && j > (unsigned)i) list[(size_t)(kMaxList - 1) * P.n + i] = j;
+                }
+            }
+            const bool again = __syncthreads_or(cnt > base + kGroupMembers);
+            if (threadIdx.x < S) {
+                const int some = min(all - base, kGroupMembers);
+                for (int q = 0; q < some; q++) sum = __fadd_rn(sum, term[q][mine]);
+            }
+            if (!again) break;
+        }
+    }
+    if (threadIdx.x < S && i0 + mine < P.n) {
         const float4 pm = pos[i0 + mine];
         const unsigned cm = cell[i0 + mine];
-        DensitySum D(list + i0 + mine);
-        if (cnt < 0) {
-            density_walk(P, pos, start, cm & ~kWide, pm, (unsigned)(i0 + mine), st, D);
-        } else {
-#pragma unroll 8
-            for (int q = 0; q < cnt; q++) D.sum = __fadd_rn(D.sum, term[q][mine]);
-            D.listed = listed;
-            D.self = itself[mine];
-        }
-        density_store(P, pos, vel, cell, rho, inv_rho, press, nbr, compute_pressure, st, i0 + mine, pm, cm, D.sum,
-                      D.listed + D.self, D.listed);
+        const bool crowded = all < 0;   // past the work cap: the particle itself only
+        if (crowded) atomicAdd(&st->crowded, 1u);
+        density_store(P, pos, vel, cell, rho, inv_rho, press, nbr, compute_pressure, st, i0 + mine, pm, cm,
+                      crowded ? 1.f : sum, crowded ? 1 : all, crowded ? 0 : listed);
     }
 }
 

@@ -1,6 +1,6 @@
-"""The density pass over states denser than its masks have room for (k_density_mask takes them in several
-rounds): members and densities against a brute-force evaluation, and a cost that grows with the
-candidates."""
+"""The density pass over states denser than its masks (k_density_mask) or its shared memory
+(k_density_group: 64 members) have room for, which take several rounds: members and densities against a
+brute-force evaluation, and a cost that grows with the candidates."""
 import time
 
 import numpy as np
@@ -22,7 +22,8 @@ STATES = {"two_rounds": (0.016, 0.02, 2.0, 2.0), "three_rounds": (0.0135, 0.02, 
 
 
 @pytest.mark.parametrize("name", list(STATES))
-@pytest.mark.parametrize("n", [20001, 77825])   # a row's records together, or one after another
+# sixteen lanes a particle, eight (up to 19,456), a row's records together (77,824), or one after another
+@pytest.mark.parametrize("n", [1716, 9729, 19456, 20001, 77825])
 def test_dense_members_and_density(gpu, name, n):
     import bubbles_gb300 as bb
     from bubbles_gb300 import scenes
@@ -65,8 +66,9 @@ def test_dense_members_and_density(gpu, name, n):
     assert (crowded > 0) == (name == "past_the_cap")
 
 
-@pytest.mark.parametrize("step,cells,kernel", [(0.85, 2.0, 2.0), (1.0, 2.5, 2.5)])
-def test_cost_grows_with_the_candidates(gpu, step, cells, kernel):
+@pytest.mark.parametrize("side,step,cells,kernel", [(60, 0.85, 2.0, 2.0), (60, 1.0, 2.5, 2.5), (21, 0.8, 2.0, 2.0),
+                                                    (25, 1.0, 3.0, 3.0)])
+def test_cost_grows_with_the_candidates(gpu, side, step, cells, kernel):
     """The work of a particle is its candidates' tests and its members' sums: a state with k times the
     members takes k times as long, here at most 1.5 k times for what the rounds repeat."""
     import bubbles_gb300 as bb
@@ -74,7 +76,7 @@ def test_cost_grows_with_the_candidates(gpu, step, cells, kernel):
     took, members = [], []
     for a, c, k in ((1.0, 2.0, 2.0), (step, cells, kernel)):
         s = 0.01
-        g = lattice((60, 60, 60), s * a)
+        g = lattice((side,) * 3, s * a)
         pos = (g - g.mean(0) + np.random.default_rng(1).uniform(-0.05, 0.05, g.shape) * s).astype(np.float32)
         sc = scenes.base_scene("pcisph", s, (1.4, 0.8, 0.8))
         sc.update(grid_spacing_scale=c, relative_kernel_radius=k)
