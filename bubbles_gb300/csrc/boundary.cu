@@ -325,9 +325,56 @@ __device__ int xiaowei(const BoundaryArgs &A, unsigned q) {
 // another out of a local array) -> 0.93 ms (a run of consecutive points per lane: the same).
 constexpr int kDiltsShared = 96, kDiltsWarps = 4, kDiltsCap = 1024;
 
+// Scattered particles (few candidates, the first point open) are told by a thread each: a warp for each
+// took 376 us for 262,144 of them, 75 now.  A block takes `turn` particles: a thread of its first warp for
+// each, its four warps for what is left; more than four when that leaves 32 blocks an SM (with 16, dense
+// particles, whose tests differ in length, waited for the last blocks: 64,000 of them 2,275 us, 2,100 so).
+constexpr unsigned kDiltsScattered = 16;
+__host__ __device__ inline int dilts_turn(int total) {
+    int turn = kDiltsWarps;
+    while (turn < 32 && total > turn * 2 * 32 * 152) turn *= 2;
+    return turn;
+}
+
 __device__ __forceinline__ float exact_distance2(float4 a, float4 b) {
     const float ex = fs(a.x, b.x), ey = fs(a.y, b.y), ez = fs(a.z, b.z);
     return fa(fa(fm(ex, ex), fm(ey, ey)), fm(ez, ez));
+}
+
+__device__ __forceinline__ float4 dilts_point(const BoundaryArgs &A, float4 p, const float *spoke, int u, int v) {
+    const float su = spoke[u], cu = spoke[65 + u], sv = spoke[130 + v], cv = spoke[195 + v], rad = A.d_rad;
+    return make_float4(fa(fm(fm(su, cv), rad), p.x), fa(fm(fm(su, sv), rad), p.y), fa(fm(cu, rad), p.z), 0.f);
+}
+
+// True when particle q has few candidates in its 27 cells and none of them holds the first point: it is
+// on the boundary.
+__device__ bool dilts_scattered(const BoundaryArgs &A, unsigned q, const float *spoke) {
+    const float4 pi = A.pos[q];
+    unsigned bad = 0, candidates = 0;
+    int u[3];
+    coords(A.g, grid_hash(A.g, pi, A.iz, &bad), u);
+    const int x0 = max(u[0] - 1, 0), x1 = min(u[0] + 1, A.g.nx - 1);
+    unsigned b[9], e[9];   // rows of three cells
+#pragma unroll
+    for (int r = 0; r < 9; r++) {
+        const int j = u[1] - 1 + r / 3, k = u[2] - 1 + r % 3;
+        b[r] = e[r] = 0;
+        if (j >= 0 && j < A.g.ny && k >= 0 && k < A.g.nz) {
+            b[r] = A.start[linear(A.g, x0, j, k)];
+            e[r] = A.start[linear(A.g, x1, j, k) + 1u];
+        }
+        candidates += e[r] - b[r];
+    }
+    if (candidates > kDiltsScattered) return false;
+    const float4 pt = dilts_point(A, pi, spoke, 0, 0);
+    bool open = true;
+#pragma unroll
+    for (int r = 0; r < 9; r++)
+        for (unsigned s = b[r]; s < e[r]; s++) {
+            const float4 pj = A.pos[s];
+            if (s != q && !(exact_distance2(pi, pj) > A.d_lim2) && exact_distance2(pj, pt) <= A.d_rad2) open = false;
+        }
+    return open;
 }
 
 __device__ int dilts(const BoundaryArgs &A, unsigned q, const float *spoke, float4 *near) {
@@ -339,24 +386,33 @@ __device__ int dilts(const BoundaryArgs &A, unsigned q, const float *spoke, floa
     int u[3];
     coords(A.g, grid_hash(A.g, pi, A.iz, &bad), u);
     __syncwarp();   // the warp's previous particle is done with `near`
-    for (int j = max(u[1] - 1, 0); j <= min(u[1] + 1, A.g.ny - 1); j++)
-        for (int i = max(u[0] - 1, 0); i <= min(u[0] + 1, A.g.nx - 1); i++)
-            for (int k = max(u[2] - 1, 0); k <= min(u[2] + 1, A.g.nz - 1); k++) {
-                const unsigned nb = linear(A.g, i, j, k), e = A.start[nb + 1];
-                for (unsigned s = A.start[nb]; s < e && n < kDiltsCap; s += 32u) {
-                    const unsigned t = s + (unsigned)lane;
-                    float4 pj = pi;
-                    bool hit = t < e && t != q;
-                    if (hit) {
-                        pj = A.pos[t];
-                        hit = !(exact_distance2(pi, pj) > A.d_lim2);
-                    }
-                    const unsigned m = __ballot_sync(full, hit);
-                    const int at = n + __popc(m & ((1u << lane) - 1u));
-                    if (hit && at < kDiltsShared) near[at] = pj;
-                    n = min(n + __popc(m), kDiltsCap);
-                }
+    // a cell's slots per lane, in walk order; then the cells that hold any, one after another
+    unsigned b = 0, len = 0;
+    if (lane < 27) {
+        const int j = u[1] - 1 + lane / 9, i = u[0] - 1 + lane / 3 % 3, k = u[2] - 1 + lane % 3;
+        if (i >= 0 && i < A.g.nx && j >= 0 && j < A.g.ny && k >= 0 && k < A.g.nz) {
+            const unsigned nb = linear(A.g, i, j, k);
+            b = A.start[nb];
+            len = A.start[nb + 1] - b;
+        }
+    }
+    for (unsigned cells = __ballot_sync(full, len > 0); cells; cells &= cells - 1u) {
+        const int from = __ffs((int)cells) - 1;
+        const unsigned first = __shfl_sync(full, b, from), e = first + __shfl_sync(full, len, from);
+        for (unsigned s = first; s < e && n < kDiltsCap; s += 32u) {
+            const unsigned t = s + (unsigned)lane;
+            float4 pj = pi;
+            bool hit = t < e && t != q;
+            if (hit) {
+                pj = A.pos[t];
+                hit = !(exact_distance2(pi, pj) > A.d_lim2);
             }
+            const unsigned m = __ballot_sync(full, hit);
+            const int at = n + __popc(m & ((1u << lane) - 1u));
+            if (hit && at < kDiltsShared) near[at] = pj;
+            n = min(n + __popc(m), kDiltsCap);
+        }
+    }
     __syncwarp();
     const int nl = min(n, kDiltsShared);
     int last = 0;
@@ -364,10 +420,7 @@ __device__ int dilts(const BoundaryArgs &A, unsigned q, const float *spoke, floa
         const int p = p0 + lane, pu = p / 65, pv = p - 65 * pu;
         bool open = false;
         if (p < 65 * 65) {
-            const float su = spoke[pu], cu = spoke[65 + pu], sv = spoke[130 + pv], cv = spoke[195 + pv];
-            const float rad = A.d_rad;
-            const float4 pt = make_float4(fa(fm(fm(su, cv), rad), pi.x), fa(fm(fm(su, sv), rad), pi.y),
-                                          fa(fm(cu, rad), pi.z), 0.f);
+            const float4 pt = dilts_point(A, pi, spoke, pu, pv);
             open = !(nl > 0 && exact_distance2(near[last], pt) <= A.d_rad2);
             if (open)
                 for (int t = 0; t < nl; t++)
@@ -405,23 +458,6 @@ __global__ void k_lnm_xiaowei(BoundaryArgs A, const int *__restrict__ queue, int
     }
 }
 
-__global__ void __launch_bounds__(32 * kDiltsWarps)
-k_lnm_dilts(BoundaryArgs A, const int *__restrict__ queue, int *__restrict__ counts, int *__restrict__ out) {
-    __shared__ float4 near[kDiltsWarps][kDiltsShared];
-    __shared__ float spoke[260];
-    const int wid = threadIdx.x >> 5, total = counts[0];
-    if (blockIdx.x * kDiltsWarps >= total) return;
-    for (int k = threadIdx.x; k < 260; k += blockDim.x) spoke[k] = A.spoke[k];
-    __syncthreads();
-    for (int t = blockIdx.x * kDiltsWarps + wid; t < total; t += gridDim.x * kDiltsWarps) {
-        const unsigned q = (unsigned)queue[t];
-        if (dilts(A, q, spoke, near[wid]) > 0 && (threadIdx.x & 31) == 0) {
-            out[A.pid[q]] = 2;
-            atomicAdd(&counts[1], 1);
-        }
-    }
-}
-
 // XiaoweiBoundary / DiltsSpokeBoundary over every particle
 __global__ void k_xiaowei(BoundaryArgs A, int n, int *__restrict__ out) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -429,16 +465,48 @@ __global__ void k_xiaowei(BoundaryArgs A, int n, int *__restrict__ out) {
     out[A.pid[q]] = xiaowei(A, (unsigned)q);
 }
 
-__global__ void __launch_bounds__(32 * kDiltsWarps)
-k_dilts(BoundaryArgs A, int n, int *__restrict__ out) {
+// Dilts over every particle, or with `queue` (of counts[0] particles) as k_lnm_xiaowei.  32 registers, for
+// 16 blocks an SM: the lanes' walk of the spheres wants the warps (262,144 particles 1,050 us at 40, 975).
+__global__ void __launch_bounds__(32 * kDiltsWarps, 16)
+k_dilts(BoundaryArgs A, int n, const int *__restrict__ queue, int *__restrict__ counts, int *__restrict__ out) {
     __shared__ float4 near[kDiltsWarps][kDiltsShared];
     __shared__ float spoke[260];
-    const int wid = threadIdx.x >> 5, q = blockIdx.x * kDiltsWarps + wid;
+    __shared__ unsigned todo[32];
+    __shared__ int left;
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, total = queue ? counts[0] : n;
+    const int turn = dilts_turn(total);
+    auto tell = [&](unsigned q, bool on) {
+        if (!queue) {
+            out[A.pid[q]] = on ? 1 : 0;
+        } else if (on) {
+            out[A.pid[q]] = 2;
+            atomicAdd(&counts[1], 1);
+        }
+    };
+    if ((long long)blockIdx.x * turn >= total) return;
     for (int k = threadIdx.x; k < 260; k += blockDim.x) spoke[k] = A.spoke[k];
     __syncthreads();
-    if (q >= n) return;
-    const int b = dilts(A, (unsigned)q, spoke, near[wid]);
-    if ((threadIdx.x & 31) == 0) out[A.pid[q]] = b;
+    for (long long t0 = (long long)blockIdx.x * turn; t0 < total; t0 += (long long)gridDim.x * turn) {
+        if (wid == 0) {
+            const bool mine = lane < turn && t0 + lane < total;
+            unsigned q = 0;
+            bool done = true;
+            if (mine) {
+                q = queue ? (unsigned)queue[t0 + lane] : (unsigned)(t0 + lane);
+                done = dilts_scattered(A, q, spoke);
+                if (done) tell(q, true);
+            }
+            const unsigned rest = __ballot_sync(0xffffffffu, !done);
+            if (!done) todo[__popc(rest & ((1u << lane) - 1u))] = q;
+            if (lane == 0) left = __popc(rest);
+        }
+        __syncthreads();
+        for (int k = wid; k < left; k += kDiltsWarps) {
+            const int b = dilts(A, todo[k], spoke, near[wid]);
+            if (lane == 0) tell(todo[k], b > 0);
+        }
+        __syncthreads();   // todo and left are read
+    }
 }
 
 }  // namespace
@@ -469,12 +537,12 @@ void launch_lnm_geometric(const BoundaryArgs &A, const unsigned *cell, int n, in
     k_lnm_queue<<<blocks_for(n, 256), 256, 0, s>>>(n, cell, A.pid, level, queue, counts, out);
     // the queue's length is on the device: enough warps for all of it, at most 16 blocks an SM
     if (algorithm == 1) k_lnm_xiaowei<<<blocks_for(n, 128), 128, 0, s>>>(A, queue, counts, out);
-    else k_lnm_dilts<<<std::min(blocks_for(n, kDiltsWarps), 16 * 152), 32 * kDiltsWarps, 0, s>>>(A, queue, counts, out);
+    else k_dilts<<<std::min(blocks_for(n, kDiltsWarps), 16 * 152), 32 * kDiltsWarps, 0, s>>>(A, n, queue, counts, out);
 }
 
 void launch_boundary_test(const BoundaryArgs &A, int algorithm, int n, int *out, cudaStream_t s) {
     if (algorithm == 1) k_xiaowei<<<blocks_for(n, 128), 128, 0, s>>>(A, n, out);
-    else k_dilts<<<blocks_for(n, kDiltsWarps), 32 * kDiltsWarps, 0, s>>>(A, n, out);
+    else k_dilts<<<blocks_for(n, dilts_turn(n)), 32 * kDiltsWarps, 0, s>>>(A, n, nullptr, nullptr, out);
 }
 
 void launch_lnm(const GridDev &g, const unsigned *start, const unsigned *cell, const int *pid, int n, int delta,
