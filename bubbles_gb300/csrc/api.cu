@@ -1534,20 +1534,30 @@ bbg_status bbg_neighbor_lists(bbg_solver s, int max_per_particle, int32_t *count
         return fail(BBG_ERR_STATE, "no neighbour sets: compute the density (or a substep) after the last grid update");
     const int n = s->n;
     const size_t width = (size_t)max_per_particle;
-    // rows of a chunk of caller ids staged in the 6 x capacity words of the staging buffer
-    size_t rows = 6 * (size_t)s->capacity / (width + 1);
-    if (rows > (size_t)n) rows = (size_t)n;
+    const size_t row = std::min(width, (size_t)kMaxCandidates);   // no particle has more members
+    // rows of a chunk of caller ids staged in the 6 x capacity words of the staging buffer, or, when
+    // it is too small for one, all of them in scratch
+    size_t rows = 6 * (size_t)s->capacity / (row + 1);
     int *dc = reinterpret_cast<int *>(s->B.stage);
+    if (rows == 0) {
+        rows = (size_t)n;
+        CK(scratch_begin(s));
+        CK(scratch_get(s, rows * (row + 1), &dc));
+    }
+    if (rows > (size_t)n) rows = (size_t)n;
+    if (row < width) std::fill(ids, ids + (size_t)n * width, -1);
     for (size_t a = 0; a < (size_t)n; a += rows) {
         const size_t b = a + rows < (size_t)n ? a + rows : (size_t)n;
         int *dout = dc + (b - a);
-        launch_export_members(s->P, s->B, s->list_state, s->pid_cur, (int)a, (int)b, max_per_particle, dc, dout,
-                              s->stream);
+        launch_export_members(s->P, s->B, s->list_state, s->pid_cur, (int)a, (int)b, (int)row, dc, dout, s->stream);
         CK_LAUNCH();
         CK(cudaMemcpyAsync(counts + a, dc, sizeof(int) * (b - a), cudaMemcpyDeviceToHost, s->stream));
-        if (width)
+        if (width && row == width)
             CK(cudaMemcpyAsync(ids + a * width, dout, sizeof(int) * (b - a) * width, cudaMemcpyDeviceToHost,
                                s->stream));
+        else if (width)
+            CK(cudaMemcpy2DAsync(ids + a * width, sizeof(int) * width, dout, sizeof(int) * row, sizeof(int) * row,
+                                 b - a, cudaMemcpyDeviceToHost, s->stream));
         CK(cudaStreamSynchronize(s->stream));
     }
     return BBG_OK;
