@@ -310,9 +310,7 @@ class Solver:
         st, out = mesh(room, 2 * room)
         if st == 4:
             st, out = mesh(npt.value, ntr.value)
-        if st != N.OK:
-            N.call("bbg_marching_cubes", self.h, ctypes.byref(g), v.ctypes.data, float(iso), 0, None, None, 0,
-                   None, 0, ctypes.byref(npt), ctypes.byref(ntr))
+        N.check(st)
         for a, rows in zip(out, (npt.value, npt.value, ntr.value)):
             a.resize((rows, 3), refcheck=False)   # gives the rest back
         return out
