@@ -42,6 +42,7 @@ PPTS = (1, 2)
 TILE_ORDERS = (0, 1)
 WORKLISTS = (0, 1, 2)
 CELL_SCALES = (2.0, 2.5, 3.0)
+FEW = 77824   # up to this many particles the passes have launches of their own (bbg.h, bbg_tuning)
 
 
 def tuned_path(config):
@@ -89,15 +90,28 @@ def time_substeps(g, dt, snap, steps, warm):
     return time.perf_counter() - t0
 
 
+def acts(key, n, tuning):
+    """Whether a knob changes a launch of n particles under the other settings."""
+    if n > FEW:
+        return True
+    if key in ("batch_pd", "batch_pf"):
+        return tuning["batch_worklist"] == 2   # the persistent batch passes
+    return key not in ("batch_np", "particles_per_thread")
+
+
 def tune_launches(g, dt, snap, steps, warm, log):
     best = dict(g.tuning())
     best_t = time_substeps(g, dt, snap, steps, warm)
     log.append({"tuning": dict(best), "seconds": best_t})
     knobs = [("block_size", BLOCKS), ("batch_pf", BATCHES), ("batch_pd", BATCHES),
              ("batch_np", BATCHES), ("particles_per_thread", PPTS), ("tile_order", TILE_ORDERS)]
-    if isinstance(g, BatchSolver):
+    batch = isinstance(g, BatchSolver)
+    if batch:
         knobs.append(("batch_worklist", WORKLISTS))
     for key, values in knobs:
+        # (a single scene has no work list, whatever the field says)
+        if not acts(key, g.n, dict(best, batch_worklist=best["batch_worklist"] if batch else 0)):
+            continue
         for v in values:
             if v == best[key]:
                 continue

@@ -470,13 +470,16 @@ bbg_status bbg_marching_cubes(bbg_solver s, const bbg_sdf_grid *grid, const floa
  * sorted particles), how many members' records a thread requests together in the
  * non-pressure, predicted-density and pressure-force passes.
  * Results do not depend on them (bit for bit); bubbles_gb300.autotune measures and picks
- * them. */
+ * them.  Few particles have launches of their own: up to 77,824 the batch_* fields (but for
+ * batch_pd and batch_pf with batch_worklist 2) and particles_per_thread are kept and have
+ * no effect, and up to 19,456 in a single scene block_size and tile_order act on the
+ * non-pressure pass alone. */
 typedef struct {
     int block_size;      /* 64, 128 (default) or 256 */
     int batch_np;        /* 2, 4 (default) or 8 */
     int batch_pd;
     int batch_pf;
-    int prune;           /* 0 or 1; no effect (the density pass filters all 27 cells' candidates) */
+    int prune;           /* 0 or 1; reserved, no effect (the density pass filters all candidates) */
     int particles_per_thread;  /* predicted-density and pressure-force passes: 1 (default) or 2 */
     int tile_order;      /* member-walking passes: 0 (default) block b takes tile b; 1 blocks
                             b, b + S, b + 2S, ... (S = the SM count) take consecutive tiles */
