@@ -116,6 +116,10 @@ struct StepState {
                                          // density pass, of the pressure-force pass after it
 };
 
+// SMs of a GB300: the lines between kernels for few and many particles (grids that fill the chip ask
+// the device).
+constexpr int kSms = 152;
+
 // Work caps that keep a degenerate state (e.g. a blown-up simulation that piles particles
 // into a few cells) from turning the per-cell rank and the candidate search quadratic:
 // a cell with more than kRankCap particles keeps its arrival order instead of the order

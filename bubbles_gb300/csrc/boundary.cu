@@ -332,7 +332,7 @@ constexpr int kDiltsShared = 96, kDiltsWarps = 4, kDiltsCap = 1024;
 constexpr unsigned kDiltsScattered = 16;
 __host__ __device__ inline int dilts_turn(int total) {
     int turn = kDiltsWarps;
-    while (turn < 32 && total > turn * 2 * 32 * 152) turn *= 2;
+    while (turn < 32 && total > turn * 2 * 32 * kSms) turn *= 2;
     return turn;
 }
 
@@ -537,7 +537,7 @@ void launch_lnm_geometric(const BoundaryArgs &A, const unsigned *cell, int n, in
     k_lnm_queue<<<blocks_for(n, 256), 256, 0, s>>>(n, cell, A.pid, level, queue, counts, out);
     // the queue's length is on the device: enough warps for all of it, at most 16 blocks an SM
     if (algorithm == 1) k_lnm_xiaowei<<<blocks_for(n, 128), 128, 0, s>>>(A, queue, counts, out);
-    else k_dilts<<<std::min(blocks_for(n, kDiltsWarps), 16 * 152), 32 * kDiltsWarps, 0, s>>>(A, n, queue, counts, out);
+    else k_dilts<<<std::min(blocks_for(n, kDiltsWarps), 16 * kSms), 32 * kDiltsWarps, 0, s>>>(A, n, queue, counts, out);
 }
 
 void launch_boundary_test(const BoundaryArgs &A, int algorithm, int n, int *out, cudaStream_t s) {

@@ -452,8 +452,8 @@ k_mlp_train(int batch, const float4 *__restrict__ bx, const float *__restrict__ 
 
 // Adam on the FP32 master parameters (bias corrections from the device step counter); the
 // gradient is the sum of the training blocks' rows in block order, the batch loss the sum
-// of their partial losses in block order (by a block of its own).  A warp a block: the 142 warps
-// on 142 SMs, 16 rows of a parameter requested together.
+// of their partial losses in block order (by a block of its own).  A warp a block: 143 for the
+// 4,545 parameters, on as many SMs, 16 rows of a parameter requested together.
 __global__ void k_mlp_adam(float *__restrict__ theta, const float *__restrict__ gpart, int rows,
                            const double *__restrict__ lpart, double *__restrict__ loss, float *__restrict__ m1,
                            float *__restrict__ m2, const unsigned *__restrict__ step, float lr, float beta1,

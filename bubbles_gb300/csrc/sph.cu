@@ -1,5 +1,5 @@
 // sph.cu -- neighbour-sum passes of the 3D SPH / PCISPH step (FP32, one thread per
-// particle over the cell-sorted arrays).
+// particle over the cell-sorted arrays; several lanes per particle for the fewest, kGroup16).
 //
 // Neighbour sets follow the reference buckets: j is a neighbour of i when
 // IsWithinStd(|x_i - x_j|, h) holds at the positions of the last grid update
@@ -59,15 +59,15 @@ constexpr int kPfWlMinBlocks = BBG_PFWL_MIN_BLOCKS * kTile / kMaxTile;
 #ifndef BBG_DENSITY_MIN_BLOCKS
 #define BBG_DENSITY_MIN_BLOCKS 8
 #endif
-// density pass: 64 registers (measured at 1M particles: 8 and 10 blocks the same, 12 spills)
+// density pass: at most 64 registers (it takes 56, 9 blocks an SM; capped for 12 it spills)
 constexpr int kDensityMinBlocks = BBG_DENSITY_MIN_BLOCKS * kTile / kMaxTile;
 
 // Up to this many particles the member passes are bound by the latency of each particle's dependent
-// loads, with few warps an SM to hide it: kernels that request more of them together, at up to
-// 128 registers, so four blocks of 128 an SM, and one wave of 152 SMs is the line.  A
-// substep of 19,720 particles, 8 corrector iterations: 218 -> 193 us; 65,600: 222 -> 208; 5,814, 1
+// loads, with few warps an SM to hide it: kernels that request more of them together (the compiler
+// takes 90 to 103 registers: five blocks of 128 an SM, four at the most).  The line is one wave of four
+// blocks an SM.  A substep of 19,720 particles, 8 corrector iterations: 218 -> 193 us; 65,600: 222 -> 208; 5,814, 1
 // iteration: 79 -> 71; past the line they lose (122,500: 271 -> 341).
-constexpr int kFew = 152 * 4 * kTile;
+constexpr int kFew = kSms * 4 * kTile;
 constexpr int kFewBatch = 16, kFewBatchPosVel = 8;   // members together (one or two records each)
 
 // a neighbour's position and velocity records
@@ -332,8 +332,8 @@ __device__ __forceinline__ int density_filter(const Params &P, const unsigned *_
 //
 // Measured at 1,048,576 particles: 234 -> 149 us; 4,194,304: 866 -> 554; 262,144: 78 -> 47 (with a
 // records' launch of its own: 156, 578, 52).  The pass that tested and summed every candidate in float was bound by issue
-// slots (256 M warp instructions, 83 %); this one issues 136 M.  The filter's bound is the FMA
-// pipe (24 half2 operations per eight candidates); with float candidates it was L1, whose 128 bytes
+// slots (256 M warp instructions, 83 %); this one issues 143 M, 77 % of the slots, with L1 at 72 % and the
+// ALU at 52 % (masks and lists).  Float candidates in the filter were bound by L1, whose 128 bytes
 // a clock return 12 bytes a candidate to every lane (181 us), half of that as halves.  A warp per
 // cell that holds candidates in registers and ballots each particle's tests was slower (225 us): the
 // setup per cell, 5.5 cells a warp, costs more than the loads it saves.
@@ -380,13 +380,13 @@ k_density_mask(Params P, float4 *__restrict__ pos, float4 *__restrict__ vel, uns
 // The fewest particles: G lanes for each instead of a thread, which is one long chain of dependent loads,
 // about 216 candidates deep, on an idle chip.  The density pass takes sixteen lanes or eight,
 // the force pass, whose 29 members are the shorter chain, eight or four: as many as keep the density pass
-// within one wave of 8 blocks of 128 on 152 SMs; past it the extra instructions of splitting a
+// within one wave of 8 blocks of 128 an SM; past it the extra instructions of splitting a
 // particle cost more than the latency they hide (12,144 particles: 16 and 8 lanes 375 us for seven
 // SPH substeps, 8 and 4 lanes 340, a thread each 371; 16,384: 8 and 4 lanes 370, a thread each 375; 20,000:
 // no difference; 35,937, 4 lanes: 461 against 374).
 constexpr int kGroupThreads = 128;
 constexpr int kGroupMembers = kMaxList;   // of a particle (itself counted) in shared memory at a time
-constexpr int kGroup16 = 152 * 8 * kGroupThreads / 16;   // particles, up to
+constexpr int kGroup16 = kSms * 8 * kGroupThreads / 16;   // particles, up to
 constexpr int kGroup8 = 2 * kGroup16;
 
 // The density pass, G lanes per particle: the lanes take every G-th candidate of the particle's nine rows,

@@ -1,7 +1,8 @@
 // tile.cuh -- tiles of the neighbour passes and the neighbour lists.
 //
-// Every neighbour pass runs one thread per particle in blocks of consecutive slots of the
-// cell-sorted arrays (a "tile": the block size, 64 to 256, a tuning parameter).
+// The neighbour passes run one thread per particle in blocks of consecutive slots of the
+// cell-sorted arrays (a "tile": the block size, 64 to 256, a tuning parameter), but for the fewest
+// particles, which get several lanes each (sph.cu).
 //
 // The density pass records each particle's neighbour set (the reference bucket) as a
 // list, member-major: entry q of particle i is list[q * n + i], so entry q of 32
